@@ -1,0 +1,24 @@
+"""The gradient read-back: transposed on the device, in chunks, to the reference's file order."""
+import numpy as np
+import pytest
+
+import denise_b200 as dn
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nx,ny", [(33, 20), (1, 40), (1201, 1801)])
+@pytest.mark.parametrize("acc", ["f32", "f64"])
+def test_gradient_readback_order(nx, ny, acc):
+    """Read-back in chunks (the largest case needs two a field): every element in its place."""
+    from denise_b200 import _lib, synth
+
+    p = synth.c0_params(nx=nx, ny=ny, nt=10, fw=0, store_snapshots=1,
+                        grad_accum=_lib.ACC_F64 if acc == "f64" else _lib.ACC_F32)
+    one = np.ones((nx, ny), np.float32)
+    m = dn.Model(p, 3000 * one, 1700 * one, 2000 * one)
+    rng = np.random.default_rng(nx)
+    g = [rng.standard_normal((nx, ny)).astype(np.float32) for _ in range(3)]
+    m.set_gradient(*g)
+    for a, b in zip(m.gradient(), g):
+        np.testing.assert_array_equal(a, b)
