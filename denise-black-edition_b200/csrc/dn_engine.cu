@@ -1007,6 +1007,25 @@ static int eff_tiles(const dn_shot *s, const LaunchCfg *c)
     return ((s->p.nx + s->bx - 1) / s->bx) * ((s->p.ny + z - 1) / z);
 }
 
+// whether the stress kernel can take over the free surface of shot s: not when a source that
+// k_inject_s adds afterwards sits in row 1 (the surface condition there starts from the sum), not
+// for moment tensors (they change sxy in two rows), and not when the images reach below the grid
+static bool surf_in_stress(const dn_shot *s, int mode, const LaunchCfg *c)
+{
+    if (!c || !c->fold || !s->p.free_surf || runs_fused(s, mode)) return false;
+    if (s->p.ny < s->p.fdorder / 2 + 1) return false;
+    if (mode == 1)
+        return s->p.quelltypb < 4 || std::find(s->rec_j.begin(), s->rec_j.end(), 1) == s->rec_j.end();
+    if (s->quelltyp_last == 5) return false;
+    return c->fuse_src || s->quelltyp_last != 1 || std::find(s->src_j.begin(), s->src_j.end(), 1) == s->src_j.end();
+}
+// whether the stress kernel's receiver blocks record shot s: the velocities only (SEISMO 2-4 need
+// the stresses after the sources and the surface, and stay with k_seismo)
+static bool rec_in_stress(const dn_shot *s, int mode, const LaunchCfg *c)
+{
+    return c && c->fold && !runs_fused(s, mode) && (mode == 1 || s->p.seismo <= 1);
+}
+
 // the descriptor of shot s in mode `mode` for a batch configured as c (the configuration the
 // batch's kernels are launched with: tile rows, in-kernel sources)
 static Inst make_inst(const dn_shot *s, int mode, const LaunchCfg *c)
@@ -1139,6 +1158,9 @@ static Inst make_inst(const dn_shot *s, int mode, const LaunchCfg *c)
         I.fsrc_v = 1;
         I.fsrc_s = s->quelltyp_last == 1;
     }
+    I.ord = p.fdorder / 2;
+    I.surf_s = surf_in_stress(s, mode, c);
+    I.rec_blocks = rec_in_stress(s, mode, c) ? c->rec_blocks : 0;
     if (runs_fused(s, mode)) {
         const int R = p.fdorder / 2;
         I.pp = 1;
@@ -1315,7 +1337,6 @@ static int check_batch(dn_shot *const *shots, int n, int mode, LaunchCfg &c, con
         maxsrc = std::max(maxsrc, std::max(s->nsrc_cells, m == 1 ? s->ntr : 0));
         maxnx = std::max(maxnx, s->p.nx);
         maxtr = std::max(maxtr, s->ntr);
-        if (s->p.free_surf) c.any_surf = true;
         if (m == 1 ? s->p.quelltypb >= 4 : (s->quelltyp_last == 1 || s->quelltyp_last == 5)) c.any_src_s = true;
         if (m == 0 && s->p.store_snapshots && s->nsnap > 0) c.any_store = true;
         if (m == 1) c.any_adj = true;
@@ -1371,6 +1392,21 @@ static int check_batch(dn_shot *const *shots, int n, int mode, LaunchCfg &c, con
             }
         }
     }
+    // free surface and velocity receivers inside the same variants of the stress kernels: two of
+    // the four dependent launches of a step go, and a small batch's step is bound by them (one
+    // 600 x 300 shot 21.9 -> 15.0 us a step, one viscoelastic 2000 x 600 shot 75 -> 63 us); in the
+    // kernels of large batches the extra row test cost more than the launches (8000 x 2000 with
+    // checkpoints 6 % slower), so those keep the surface and receiver kernels
+    c.fold = c.fuse_src;
+    c.rec_blocks = 0;
+    for (int k = 0; k < n; k++) {
+        const dn_shot *s = shots[k];
+        const int m = modes ? modes[k] : mode;
+        if (s->p.free_surf && !surf_in_stress(s, m, &c)) c.any_surf = true;
+        if (rec_in_stress(s, m, &c)) c.rec_blocks = std::max(1, std::min((maxtr + 127) / 128, 16));
+        else c.any_rec = true;
+    }
+    c.s_grid = dim3(maxtiles + c.rec_blocks, n);
     c.src_grid = dim3((maxsrc + 127) / 128, n);
     c.surf_grid = dim3((maxnx + 127) / 128, n);
     c.rec_grid = dim3((maxtr + 127) / 128, n);
@@ -1660,6 +1696,8 @@ static int run_direct(dn_shot *s, int mode, int nt0, int nt1, bool zero)
         h.pp = 0;
         c.any_fused = false;
         c.any_plain = true;
+        c.any_surf = s->p.free_surf;   // its surface and receivers from their own kernels
+        c.any_rec = true;
         if (c.fuse_src && mode != 1) {   // its sources then come from the stencil kernels
             h.fsrc_v = 1;
             h.fsrc_s = s->quelltyp_last == 1;

@@ -96,6 +96,10 @@ struct Inst {
     // stress kernels (explosive, QUELLTYP 1) instead of k_inject_v / k_inject_s
     int fsrc_v, fsrc_s;
     int rec_dup;                      // two receivers share a cell: adjoint sources added in list order
+    // work folded into the stress kernels of small batches: the free surface of row 1 and its image rows (surf_s),
+    // and the velocity receivers and the NaN probe in the first rec_blocks blocks of its grid
+    int surf_s, rec_blocks;
+    int ord;                          // FDORDER / 2
     // prepared viscoelastic coefficients (the per-kernel drop-in of update_s_visc_PML_PSV,
     // which receives them): fipjp, f, g planes and d, e, dip planes per mechanism at + l * plane
     const float *pre_fipjp, *pre_f, *pre_g, *pre_d, *pre_e, *pre_dip;
@@ -159,9 +163,8 @@ __device__ __forceinline__ float DIVK(float a, float k)
 struct TileLoc {
     int i, j0, j1;
 };
-__device__ __forceinline__ bool tile_of(const Inst &I, TileLoc &t)
+__device__ __forceinline__ bool tile_of(const Inst &I, TileLoc &t, int b)
 {
-    int b = blockIdx.x;
     if (b >= I.tiles) return false;
     int tx = b % I.tiles_x, tz = b / I.tiles_x;
     t.i = tx * blockDim.x + threadIdx.x + 1;
@@ -190,7 +193,7 @@ __global__ void __maxnreg__(40) k_update_v(const Inst *__restrict__ insts, const
     const int nt = *ntb + off - I.t0;   // the instance's own time step
     if (nt < 1 || nt > I.nt) return;
     TileLoc t;
-    if (!tile_of(I, t)) return;
+    if (!tile_of(I, t, blockIdx.x)) return;
     const long long P = I.pitch;
     const int i = t.i;
     const float *__restrict__ sxx = I.sxx + i;
@@ -754,6 +757,136 @@ struct VDeriv {
 };
 
 // ===========================================================================
+// Free surface at row j = 1 (image method).  The surface part of one column:
+// surface_elastic_PML_PSV.c:60-103 and surface_visc_PML_PSV.c:60-170, shared by
+// the stress kernels (Inst::surf_s) and the surface kernels below.
+// ===========================================================================
+// vxx and vyy of row 1 in column i (origin offset o), with the x frame's CPML memory
+template <int R, bool X>
+__device__ __forceinline__ void surface_deriv(const Inst &I, int i, long long o, float &vxx, float &vyy)
+{
+    const long long P = I.pitch;
+    vxx = 0.0f, vyy = 0.0f;
+#pragma unroll
+    for (int m = 1; m <= R; m++) {
+        vxx = ADD<X>(vxx, MUL<X>(I.hc[m], SUB<X>(I.vx[o + m - 1], I.vx[o - m])));
+        vyy = ADD<X>(vyy, MUL<X>(I.hc[m], SUB<X>(I.vy[o + (m - 1) * P], I.vy[o - m * P])));
+    }
+    vxx = MUL<X>(vxx, I.dh1);
+    vyy = MUL<X>(vyy, I.dh1);
+    const int fw = I.fw, nx = I.nx;
+    if (fw > 0) {
+        if (i <= fw) {
+            const int h = i - 1;
+            float *ps = I.psi_vxxs + h;
+            float v = ADD<X>(MUL<X>(I.b_x[h], *ps), MUL<X>(I.a_x[h], vxx));
+            *ps = v;
+            vxx = ADD<X>(DIVK<X>(vxx, I.K_x[h]), v);
+        }
+        if (i >= nx - fw + 1) {
+            const int h = i - nx + 2 * fw - 1;
+            float *ps = I.psi_vxxs + h;
+            float v = ADD<X>(MUL<X>(I.b_x[h], *ps), MUL<X>(I.a_x[h], vxx));
+            *ps = v;
+            vxx = ADD<X>(DIVK<X>(vxx, I.K_x[h]), v);
+        }
+    }
+}
+
+// sxx of row 1 after the elastic surface condition
+template <int R, bool X>
+__device__ __forceinline__ float surface_sxx_el(const Inst &I, int i, long long o, float sxx)
+{
+    float vxx, vyy;
+    surface_deriv<R, X>(I, i, o, vxx, vyy);
+    const float g = I.lam[o];
+    const float fjm = MUL<X>(I.mu[o], 2.0f);   // rho*u*u*2.0 (exact doubling)
+    const float t1 = MUL<X>(DIV<X>(MUL<X>(g, g), ADD<X>(g, fjm)), vxx);
+    const float t2 = MUL<X>(g, vyy);
+    return ADD<X>(sxx, MUL<X>(-I.DT, ADD<X>(t1, t2)));
+}
+
+// sxx of row 1 after the viscoelastic surface condition; po: the column's p at row 1 (plane l
+// at + l * plane), updated in place (relaxed moduli from ws = 2 pi / TS, per-column constants
+// precomputed on the host)
+template <int R, int L, bool X>
+__device__ __forceinline__ float surface_sxx_vi(const Inst &I, int i, long long o, float sxx0, float *po)
+{
+    float vxx, vyy;
+    surface_deriv<R, X>(I, i, o, vxx, vyy);
+    const float mu = I.s_mu[i - 1], pi = I.s_pi[i - 1], taus = I.s_taus[i - 1], taup = I.s_taup[i - 1];
+    const float DT = I.DT, dthalbe = I.dthalbe;
+    const float fL = (float)L;
+    float sump = 0.0f;
+#pragma unroll
+    for (int l = 0; l < L; l++) sump = ADD<X>(sump, po[l * I.plane]);
+    const float fjm = F(DMUL(DMUL((double)mu, 2.0), DADD(1.0, (double)MUL<X>(fL, taus))));
+    const float g = F(DMUL((double)pi, DADD(1.0, (double)MUL<X>(fL, taup))));
+    const float gf = SUB<X>(g, fjm);
+    const float DTgf = MUL<X>(DT, gf);
+    float a = -DIV<X>(MUL<X>(MUL<X>(DTgf, gf), vxx), g);
+    a = SUB<X>(a, MUL<X>(DTgf, vyy));
+    a = SUB<X>(a, MUL<X>(dthalbe, sump));
+    float sxx = ADD<X>(sxx0, a);
+    sump = 0.0f;
+    const float djm = F(DMUL(DMUL(2.0, (double)mu), (double)taus));
+    const float e = MUL<X>(pi, taup);
+    const float de = SUB<X>(djm, e);
+    const double fg1 = DSUB((double)DIV<X>(fjm, g), 1.0);
+#pragma unroll
+    for (int l = 0; l < L; l++) {
+        const float bjm = I.s_bjm[l];
+        const double inner = DSUB(DMUL(DMUL((double)de, fg1), (double)vxx), (double)MUL<X>(de, vyy));
+        const float pv = F(DADD((double)po[l * I.plane], DMUL((double)bjm, inner)));
+        po[l * I.plane] = pv;
+        sump = ADD<X>(sump, pv);
+    }
+    return ADD<X>(sxx, MUL<X>(dthalbe, sump));
+}
+
+// the same out of line, for the stress kernels: inlined into their row loops it costs registers
+// that every row would pay for with spills
+template <int R, bool X>
+__device__ __noinline__ float surface_sxx_el_call(const Inst &I, int i, long long o, float sxx)
+{
+    return surface_sxx_el<R, X>(I, i, o, sxx);
+}
+template <int R, int L, bool X>
+__device__ __noinline__ float surface_sxx_vi_call(const Inst &I, int i, long long o, float sxx, float *po)
+{
+    return surface_sxx_vi<R, L, X>(I, i, o, sxx, po);
+}
+
+// the image rows of row j <= R + 1 above the surface: syy(2 - j) = -syy(j), sxy(1 - j) = -sxy(j)
+template <int R>
+__device__ __forceinline__ void surface_images(const Inst &I, int j, long long o, float syy, float sxy)
+{
+    const long long P = I.pitch;
+    if (j > 1) I.syy[o - 2 * (j - 1) * P] = -syy;
+    if (j <= R) I.sxy[o - (2 * j - 1) * P] = -sxy;
+}
+
+// Velocity receivers (seismo_ssg.c, SEISMO 1: sample nt of every trace) and the psv.c:99 NaN
+// probe on vy[NY/2][NX/2], by block rb of nrb blocks of the stress kernel: the velocities of
+// step nt are final once the velocity kernel (and k_inject_v) has run.
+__device__ __forceinline__ void record_velocities(const Inst &I, int nt, int rb, int nrb)
+{
+    const long long P = I.pitch;
+    if (rb == 0 && threadIdx.x == 0) {
+        const float v = I.vy[(long long)(I.ny / 2) * P + I.nx / 2];
+        if (isnan(v)) atomicOr(I.flag, 1);
+    }
+    if (I.mode == 1 || !I.seismo) return;
+    const long long slab = (long long)I.nt * I.ntr;
+    for (int itr = rb * blockDim.x + threadIdx.x; itr < I.ntr; itr += nrb * blockDim.x) {
+        const long long o = (long long)I.rec_j[itr] * P + I.rec_i[itr];
+        const long long s = (long long)(nt - 1) * I.ntr + itr;
+        I.sec[s] = I.vx[o];
+        I.sec[slab + s] = I.vy[o];
+    }
+}
+
+// ===========================================================================
 // Elastic stress update: update_s_elastic_PML_PSV.c (case 8 = :335-476),
 // with f = rho vs^2 and g = rho (vp^2 - 2 vs^2) precomputed per cell
 // (:442-444) and the double-promoted 2.0*f*vxx terms (:454-456).
@@ -766,7 +899,7 @@ __global__ void __launch_bounds__(256, 4) k_update_s_el(const Inst *__restrict__
     const int nt = *ntb + off - I.t0;   // the instance's own time step
     if (nt < 1 || nt > I.nt) return;
     TileLoc t;
-    if (!tile_of(I, t)) return;
+    if (!tile_of(I, t, blockIdx.x)) return;
     const long long P = I.pitch;
     const int i = t.i;
     float hc[R + 1];
@@ -913,7 +1046,14 @@ __global__ void __launch_bounds__(128, DN_S2_MINB) k_update_s_el2(const Inst *__
     if (I.pp) return;   // the fused step handles this instance
     const int nt = *ntb + off - I.t0;   // the instance's own time step
     if (nt < 1 || nt > I.nt) return;
-    const int b = blockIdx.x;
+    int b = blockIdx.x;
+    if constexpr (SRC) {   // the first rec_blocks blocks record the receivers
+        b -= I.rec_blocks;
+        if (b < 0) {
+            record_velocities(I, nt, blockIdx.x, I.rec_blocks);
+            return;
+        }
+    }
     if (b >= I.tiles) return;
     const int bxw = 2 * blockDim.x;
     const int tx = b % I.tiles_x, tz = b / I.tiles_x;
@@ -927,6 +1067,7 @@ __global__ void __launch_bounds__(128, DN_S2_MINB) k_update_s_el2(const Inst *__
     for (int m = 1; m <= R; m++) hc[m] = I.hc[m];
     const float dhi = I.dhi_el;
     const bool srcs = SRC && I.fsrc_s && src_in_columns(I, i0, two, j0, j1);
+    const int jsurf = SRC && I.surf_s ? R + 1 : 0;   // the last row with an image above the surface
     for (int j = j0; j <= j1; j++) {
         const long long o = (long long)j * P + i0;
         {
@@ -956,6 +1097,15 @@ __global__ void __launch_bounds__(128, DN_S2_MINB) k_update_s_el2(const Inst *__
             nsyy.y = F(DADD((double)s_yy.y, DADD((double)gdiv.y, DMUL(f2y, (double)vyy.y))));
         }
         if (srcs) src_explosive_pair(I, i0, two, j, nt, nsxx, nsyy);
+        if (SRC && j <= jsurf) {
+            if (j == 1) {
+                nsyy = make_float2(0.0f, 0.0f);
+                nsxx.x = surface_sxx_el_call<R, X>(I, i0, o, nsxx.x);
+                if (two) nsxx.y = surface_sxx_el_call<R, X>(I, i0 + 1, o + 1, nsxx.y);
+            }
+            surface_images<R>(I, j, o, nsyy.x, nsxy.x);
+            if (two) surface_images<R>(I, j, o + 1, nsyy.y, nsxy.y);
+        }
         st2(I.sxy + o, nsxy, two);
         st2(I.sxx + o, nsxx, two);
         st2(I.syy + o, nsyy, two);
@@ -974,8 +1124,16 @@ __global__ void __launch_bounds__(256, 3) k_update_s_vi(const Inst *__restrict__
     const Inst &I = insts[blockIdx.y];
     const int nt = *ntb + off - I.t0;   // the instance's own time step
     if (nt < 1 || nt > I.nt) return;
+    int b = blockIdx.x;
+    if constexpr (SRC) {   // the first rec_blocks blocks record the receivers
+        b -= I.rec_blocks;
+        if (b < 0) {
+            record_velocities(I, nt, blockIdx.x, I.rec_blocks);
+            return;
+        }
+    }
     TileLoc t;
-    if (!tile_of(I, t)) return;
+    if (!tile_of(I, t, b)) return;
     const long long P = I.pitch;
     const long long PL = I.plane;
     const int i = t.i;
@@ -1039,6 +1197,7 @@ __global__ void __launch_bounds__(256, 3) k_update_s_vi(const Inst *__restrict__
         }
     };
     const bool srcs = SRC && I.fsrc_s && src_in_columns(I, i, false, t.j0, t.j1);
+    const int jsurf = SRC && I.surf_s ? R + 1 : 0;   // the last row with an image above the surface
     fetch(t.j0);
     for (int j = t.j0; j <= t.j1; j++) {
         D.advance(j);
@@ -1097,12 +1256,23 @@ __global__ void __launch_bounds__(256, 3) k_update_s_vi(const Inst *__restrict__
             sump = ADD<X>(sump, pv);
             sumq = ADD<X>(sumq, qv);
         }
-        sxyp[o] = ADD<X>(sxy, MUL<X>(dthalbe, sumr));
+        const float fsxy = ADD<X>(sxy, MUL<X>(dthalbe, sumr));
+        sxyp[o] = fsxy;
         float fsxx = ADD<X>(sxx, MUL<X>(dthalbe, sump)), fsyy = ADD<X>(syy, MUL<X>(dthalbe, sumq));
         if (srcs)
             for (int c = 0; c < I.nsrc_cells; c++)
                 if (I.src_cell_j[c] == j && I.src_cell_i[c] == i)
                     fz_explosive(I, I.src_cell_start[c], I.src_cell_count[c], nt, fsxx, fsyy);
+        if (SRC && j <= jsurf) {
+            if (j == 1) {
+                fsyy = 0.0f;
+#pragma unroll
+                for (int l = 0; l < L; l++) qp[o + l * PL] = 0.0f;
+                fsxx = surface_sxx_vi_call<R, L, X>(I, i, o + i, fsxx, pp_ + o);
+            }
+            if (j > 1) syyp[o - 2 * (j - 1) * P] = -fsyy;
+            if (j <= R) sxyp[o - (2 * j - 1) * P] = -fsxy;
+        }
         sxxp[o] = fsxx;
         syyp[o] = fsyy;
         D.shift();
@@ -1114,6 +1284,13 @@ __global__ void __launch_bounds__(256, 3) k_update_s_vi(const Inst *__restrict__
 // pressure source psource.c:41-53 (mode 1, QUELLTYPB >= 4) and the moment
 // tensor source msource.c:27-41 (QUELLTYP == 5, forward modes).
 // ===========================================================================
+// a stress source added below a surface that the stress kernel has already mirrored: the image
+// row of syy follows (rows 2 to R + 1; shots with such a source in row 1 keep the surface kernel)
+__device__ __forceinline__ void inject_image(const Inst &I, int j, long long o, float syy)
+{
+    if (I.surf_s && j >= 2 && j <= I.ord + 1) I.syy[o - 2 * (j - 1) * (long long)I.pitch] = -syy;
+}
+
 static __global__ void k_inject_s(const Inst *__restrict__ insts, const int *__restrict__ ntb, int off)
 {
     const Inst &I = insts[blockIdx.y];
@@ -1130,7 +1307,9 @@ static __global__ void k_inject_s(const Inst *__restrict__ insts, const int *__r
             const long long o = (long long)I.rec_j[l] * P + I.rec_i[l];
             const float s = I.res_p[(long long)l * I.nt + (nt - 1)];
             I.sxx[o] = __fadd_rn(I.sxx[o], s);
-            I.syy[o] = __fadd_rn(I.syy[o], s);
+            const float syy = __fadd_rn(I.syy[o], s);
+            I.syy[o] = syy;
+            inject_image(I, I.rec_j[l], o, syy);
         }
         return;
     }
@@ -1152,6 +1331,7 @@ static __global__ void k_inject_s(const Inst *__restrict__ insts, const int *__r
             }
             I.sxx[o] = sxx;
             I.syy[o] = syy;
+            inject_image(I, I.src_cell_j[c], o, syy);
         }
     } else if (I.quelltyp_last == 5) {
         // neighbouring moment-tensor sources touch overlapping cells: one thread, list order
@@ -1177,129 +1357,48 @@ static __global__ void k_inject_s(const Inst *__restrict__ insts, const int *__r
     }
 }
 
-// ===========================================================================
-// Free surface at row j = 1 (image method), surface_elastic_PML_PSV.c:29-103.
-// ===========================================================================
+// The surface kernels run for the instances whose stress kernel leaves the surface to them
+// (Inst::surf_s 0: the variants without it, and sources that k_inject_s adds to row 1).
 template <int R, bool X>
 __global__ void k_surface_el(const Inst *__restrict__ insts, const int *__restrict__ ntb, int off)
 {
     const Inst &I = insts[blockIdx.y];
-    if (I.pp) return;   // the fused step handles this instance
+    if (I.pp || I.surf_s) return;   // the fused step or the stress kernel handles this instance
     const int nt = *ntb + off - I.t0;   // the instance's own time step
     if (nt < 1 || nt > I.nt || !I.free_surf) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     if (i > I.nx) return;
     const long long P = I.pitch;
-    const int j = 1;
-    const long long o = (long long)j * P + i;
+    const long long o = P + i;   // row 1
     I.syy[o] = 0.0f;
-    float vxx = 0.0f, vyy = 0.0f;
 #pragma unroll
     for (int m = 1; m <= R; m++) {
         I.syy[o - m * P] = -I.syy[o + m * P];
         I.sxy[o - m * P] = -I.sxy[o + (m - 1) * P];
-        vxx = ADD<X>(vxx, MUL<X>(I.hc[m], SUB<X>(I.vx[o + m - 1], I.vx[o - m])));
-        vyy = ADD<X>(vyy, MUL<X>(I.hc[m], SUB<X>(I.vy[o + (m - 1) * P], I.vy[o - m * P])));
     }
-    vxx = MUL<X>(vxx, I.dh1);
-    vyy = MUL<X>(vyy, I.dh1);
-    const int fw = I.fw, nx = I.nx;
-    if (fw > 0) {
-        if (i <= fw) {
-            const int h = i - 1;
-            float *ps = I.psi_vxxs + (long long)(j - 1) * 2 * fw + h;
-            float v = ADD<X>(MUL<X>(I.b_x[h], *ps), MUL<X>(I.a_x[h], vxx));
-            *ps = v;
-            vxx = ADD<X>(DIVK<X>(vxx, I.K_x[h]), v);
-        }
-        if (i >= nx - fw + 1) {
-            const int h = i - nx + 2 * fw - 1;
-            float *ps = I.psi_vxxs + (long long)(j - 1) * 2 * fw + h;
-            float v = ADD<X>(MUL<X>(I.b_x[h], *ps), MUL<X>(I.a_x[h], vxx));
-            *ps = v;
-            vxx = ADD<X>(DIVK<X>(vxx, I.K_x[h]), v);
-        }
-    }
-    const float g = I.lam[o];
-    const float fjm = MUL<X>(I.mu[o], 2.0f);   // rho*u*u*2.0 (exact doubling)
-    const float t1 = MUL<X>(DIV<X>(MUL<X>(g, g), ADD<X>(g, fjm)), vxx);
-    const float t2 = MUL<X>(g, vyy);
-    I.sxx[o] = ADD<X>(I.sxx[o], MUL<X>(-I.DT, ADD<X>(t1, t2)));
+    I.sxx[o] = surface_sxx_el<R, X>(I, i, o, I.sxx[o]);
 }
 
-// ===========================================================================
-// Viscoelastic free surface, surface_visc_PML_PSV.c:60-170 (relaxed moduli
-// from ws = 2 pi / TS, per-column constants precomputed on the host).
-// ===========================================================================
 template <int R, int L, bool X>
 __global__ void k_surface_vi(const Inst *__restrict__ insts, const int *__restrict__ ntb, int off)
 {
     const Inst &I = insts[blockIdx.y];
+    if (I.surf_s) return;   // the stress kernel handles this instance
     const int nt = *ntb + off - I.t0;   // the instance's own time step
     if (nt < 1 || nt > I.nt || !I.free_surf) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     if (i > I.nx) return;
     const long long P = I.pitch;
-    const int j = 1;
-    const long long o = (long long)j * P + i;
+    const long long o = P + i;   // row 1
     I.syy[o] = 0.0f;
 #pragma unroll
     for (int l = 0; l < L; l++) I.q[o + l * I.plane] = 0.0f;
-    float vxx = 0.0f, vyy = 0.0f;
 #pragma unroll
     for (int m = 1; m <= R; m++) {
         I.syy[o - m * P] = -I.syy[o + m * P];
         I.sxy[o - m * P] = -I.sxy[o + (m - 1) * P];
-        vxx = ADD<X>(vxx, MUL<X>(I.hc[m], SUB<X>(I.vx[o + m - 1], I.vx[o - m])));
-        vyy = ADD<X>(vyy, MUL<X>(I.hc[m], SUB<X>(I.vy[o + (m - 1) * P], I.vy[o - m * P])));
     }
-    vxx = MUL<X>(vxx, I.dh1);
-    vyy = MUL<X>(vyy, I.dh1);
-    const int fw = I.fw, nx = I.nx;
-    if (fw > 0) {
-        if (i <= fw) {
-            const int h = i - 1;
-            float *ps = I.psi_vxxs + (long long)(j - 1) * 2 * fw + h;
-            float v = ADD<X>(MUL<X>(I.b_x[h], *ps), MUL<X>(I.a_x[h], vxx));
-            *ps = v;
-            vxx = ADD<X>(DIVK<X>(vxx, I.K_x[h]), v);
-        }
-        if (i >= nx - fw + 1) {
-            const int h = i - nx + 2 * fw - 1;
-            float *ps = I.psi_vxxs + (long long)(j - 1) * 2 * fw + h;
-            float v = ADD<X>(MUL<X>(I.b_x[h], *ps), MUL<X>(I.a_x[h], vxx));
-            *ps = v;
-            vxx = ADD<X>(DIVK<X>(vxx, I.K_x[h]), v);
-        }
-    }
-    const float mu = I.s_mu[i - 1], pi = I.s_pi[i - 1], taus = I.s_taus[i - 1], taup = I.s_taup[i - 1];
-    const float DT = I.DT, dthalbe = I.dthalbe;
-    const float fL = (float)L;
-    float sump = 0.0f;
-#pragma unroll
-    for (int l = 0; l < L; l++) sump = ADD<X>(sump, I.p[o + l * I.plane]);
-    const float fjm = F(DMUL(DMUL((double)mu, 2.0), DADD(1.0, (double)MUL<X>(fL, taus))));
-    const float g = F(DMUL((double)pi, DADD(1.0, (double)MUL<X>(fL, taup))));
-    const float gf = SUB<X>(g, fjm);
-    const float DTgf = MUL<X>(DT, gf);
-    float a = -DIV<X>(MUL<X>(MUL<X>(DTgf, gf), vxx), g);
-    a = SUB<X>(a, MUL<X>(DTgf, vyy));
-    a = SUB<X>(a, MUL<X>(dthalbe, sump));
-    float sxx = ADD<X>(I.sxx[o], a);
-    sump = 0.0f;
-    const float djm = F(DMUL(DMUL(2.0, (double)mu), (double)taus));
-    const float e = MUL<X>(pi, taup);
-    const float de = SUB<X>(djm, e);
-    const double fg1 = DSUB((double)DIV<X>(fjm, g), 1.0);
-#pragma unroll
-    for (int l = 0; l < L; l++) {
-        const float bjm = I.s_bjm[l];
-        const double inner = DSUB(DMUL(DMUL((double)de, fg1), (double)vxx), (double)MUL<X>(de, vyy));
-        const float pv = F(DADD((double)I.p[o + l * I.plane], DMUL((double)bjm, inner)));
-        I.p[o + l * I.plane] = pv;
-        sump = ADD<X>(sump, pv);
-    }
-    I.sxx[o] = ADD<X>(sxx, MUL<X>(dthalbe, sump));
+    I.sxx[o] = surface_sxx_vi<R, L, X>(I, i, o, I.sxx[o], I.p + o);
 }
 
 // ===========================================================================
@@ -1313,6 +1412,7 @@ __global__ void k_seismo(const Inst *__restrict__ insts, const int *__restrict__
     const Inst &I = insts[blockIdx.y];
     const int nt = *ntb + off - I.t0;   // the instance's own time step
     if (nt < 1 || nt > I.nt) return;
+    if (I.rec_blocks) return;   // recorded by the stress kernel
     const long long P = I.pitch;
     // the buffers holding step nt's result (the second set after odd-distance steps of a fused instance)
     const bool alt = I.pp && ((I.nt - nt) & 1) != 0;

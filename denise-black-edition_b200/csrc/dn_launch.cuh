@@ -12,6 +12,7 @@ namespace dn {
 
 struct LaunchCfg {
     dim3 tile_grid, src_grid, surf_grid, rec_grid;
+    dim3 s_grid;      // grid of the stress kernels: rec_blocks receiver blocks, then the tiles
     int bx;
     int auto_zch;     // rows per tile of the shots whose tiles the batch chooses (0: their own)
     int R, L;
@@ -21,7 +22,11 @@ struct LaunchCfg {
     bool vpipe; // velocity update by the warp-specialised copy pipeline (k_update_v_pipe)
     dim3 vgrid; // its grid: strips of VP_W columns x vsh rows per instance
     int vsh;
-    bool any_surf, any_src_s, any_store, any_adj, any_rec;
+    bool fold;        // the stress kernels can take the free surface and the velocity receivers
+    int rec_blocks;   // receiver blocks of their grid
+    bool any_surf;    // k_surface_* still has work
+    bool any_rec;     // k_seismo still has work
+    bool any_src_s, any_store, any_adj;
     bool fuse_src;       // forward sources applied inside the velocity / stress kernels (Inst::fsrc_*)
     bool need_inject_v;  // k_inject_v still has work (adjoint forces, or sources not in the kernels)
     bool any_fused;   // some instance runs the fused elastic step (Inst::pp)
