@@ -160,6 +160,7 @@ struct dn_shot {
     float *psi[9];
     char *dacq = nullptr;          // source / receiver tables + signals
     int nsrc_cells;
+    std::vector<int> cell_src;     // first source of each cell
     int *d_cell_i, *d_cell_j, *d_cell_start, *d_cell_count, *d_perm, *d_src_type, *d_rec_i, *d_rec_j;
     double *d_nsin, *d_cos;
     float *d_signals;
@@ -827,6 +828,7 @@ extern "C" int dn_shot_create(dn_model *m, const dn_acq *acq, dn_shot **out)
             cj.push_back(s->src_j[l]);
             cs.push_back(k);
             cc.push_back(0);
+            s->cell_src.push_back(l);
         }
         cc.back()++;
     }
@@ -990,8 +992,9 @@ static void *acc_ptr(const dn_shot *s, int k)
     return b + 3 * a + (k - 3) * w;
 }
 
+constexpr long long SMALL_CELLS = 1300000;   // cells of a batch below which the small kernels run
 // source cells per shot up to which the stencil kernels apply the forward sources themselves
-constexpr int SRC_IN_KERNEL = 8;
+constexpr int SRC_IN_KERNEL = DN_SRC_CELLS;
 
 // a forward run (mode 0 or 2) of a shot with the second field set takes the fused step
 static bool runs_fused(const dn_shot *s, int mode) { return s->fz && (mode == 0 || mode == 2); }
@@ -1157,6 +1160,11 @@ static Inst make_inst(const dn_shot *s, int mode, const LaunchCfg *c)
     if (c && c->fuse_src && mode != 1 && !runs_fused(s, mode)) {
         I.fsrc_v = 1;
         I.fsrc_s = s->quelltyp_last == 1;
+        for (int k = 0; k < s->nsrc_cells; k++) {
+            I.sc_i[k] = s->src_i[s->cell_src[k]];
+            I.sc_j[k] = s->src_j[s->cell_src[k]];
+            I.sc_l[k] = s->cell_src[k];
+        }
     }
     I.ord = p.fdorder / 2;
     I.surf_s = surf_in_stress(s, mode, c);
@@ -1398,6 +1406,20 @@ static int check_batch(dn_shot *const *shots, int n, int mode, LaunchCfg &c, con
     // kernels of large batches the extra row test cost more than the launches (8000 x 2000 with
     // checkpoints 6 % slower), so those keep the surface and receiver kernels
     c.fold = c.fuse_src;
+    // one-row elastic batches (below 1.3 M cells): the kernels built for the shortest chain of
+    // dependent round trips; they take a column or row to lie in one CPML side at most, and every
+    // instance through the separate kernels.  Above, resident blocks count for more than the chain:
+    // three 1501 x 747 shots (3.4 M cells) took 62.0 ms with them and 45.4 with the paired kernels.
+    // DN_SMALL=0 / 1: never / whatever the size
+    {
+        const char *sm = getenv("DN_SMALL");
+        long long cells = 0;
+        for (int k = 0; k < n; k++) cells += (long long)shots[k]->p.nx * shots[k]->p.ny;
+        c.small = c.fuse_src && c.L == 0 && !c.any_fused && (sm ? strcmp(sm, "0") != 0 : cells < SMALL_CELLS);
+        for (int k = 0; k < n; k++)
+            if (shots[k]->p.nx < 2 * shots[k]->p.fw || shots[k]->p.ny < 2 * shots[k]->p.fw || shots[k]->bx > 128)
+                c.small = false;
+    }
     c.rec_blocks = 0;
     for (int k = 0; k < n; k++) {
         const dn_shot *s = shots[k];

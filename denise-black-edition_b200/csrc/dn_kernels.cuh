@@ -35,6 +35,7 @@ namespace dn {
 // "origin" pointers: element (j, i) (1-based, the reference's indices) is
 // p[j * pitch + i].
 // ---------------------------------------------------------------------------
+#define DN_SRC_CELLS 8   // source cells per shot up to which the stencil kernels apply the forward sources
 struct Inst {
     int nx, ny, nt, pitch;
     int fw, free_surf, L, mode;       // mode: 0 forward, 1 adjoint, 2 objective
@@ -100,6 +101,7 @@ struct Inst {
     // and the velocity receivers and the NaN probe in the first rec_blocks blocks of its grid
     int surf_s, rec_blocks;
     int ord;                          // FDORDER / 2
+    int sc_i[DN_SRC_CELLS], sc_j[DN_SRC_CELLS], sc_l[DN_SRC_CELLS];   // source cells and their first sources (fsrc_*)
     // prepared viscoelastic coefficients (the per-kernel drop-in of update_s_visc_PML_PSV,
     // which receives them): fipjp, f, g planes and d, e, dip planes per mechanism at + l * plane
     const float *pre_fipjp, *pre_f, *pre_g, *pre_d, *pre_e, *pre_dip;

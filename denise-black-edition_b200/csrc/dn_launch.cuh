@@ -7,6 +7,7 @@
 #include "dn_kernels_tma.cuh"
 #include "dn_kernels_vpipe.cuh"
 #include "dn_kernels_fused.cuh"
+#include "dn_kernels_small.cuh"
 
 namespace dn {
 
@@ -19,6 +20,7 @@ struct LaunchCfg {
     bool exact;
     bool tma;   // stencil kernels fed by the bulk-copy row pipeline
     bool pack;  // paired-column (FP32x2) stencil kernels, bx / 2 threads per tile
+    bool small; // the smallest elastic batches: k_update_v2_small, k_update_s_el2_small
     bool vpipe; // velocity update by the warp-specialised copy pipeline (k_update_v_pipe)
     dim3 vgrid; // its grid: strips of VP_W columns x vsh rows per instance
     int vsh;

@@ -19,6 +19,7 @@ void launch_step_R(const LaunchCfg &c, cudaStream_t st, const Inst *d, const int
         if (c.vpipe) k_update_v_pipe<R, X><<<c.vgrid, VP_THREADS, vpipe_smem_bytes(), st>>>(d, ntb, off, c.vsh);
         else if (c.tma)
             k_update_v_tma<R, X><<<c.tile_grid, TMA_W, pipe_smem_bytes<QV>(slot_floats_v()), st>>>(d, ntb, off);
+        else if (c.small) launch_pdl(k_update_v2_small<R, X>, c.tile_grid, c.bx / 2, st, d, ntb, off);
         else if (c.pack && c.fuse_src) k_update_v2<R, X, true><<<c.tile_grid, c.bx / 2, 0, st>>>(d, ntb, off);
         else if (c.pack) k_update_v2<R, X><<<c.tile_grid, c.bx / 2, 0, st>>>(d, ntb, off);
         else k_update_v<R, X><<<c.tile_grid, c.bx, 0, st>>>(d, ntb, off);
@@ -35,6 +36,7 @@ void launch_step_R(const LaunchCfg &c, cudaStream_t st, const Inst *d, const int
     } else if (c.L == 0) {
         if (c.tma)
             k_update_s_el_tma<R, X><<<c.tile_grid, TMA_W, pipe_smem_bytes<QS_EL>(slot_floats_s_el()), st>>>(d, ntb, off);
+        else if (c.small) launch_pdl(k_update_s_el2_small<R, X>, c.s_grid, c.bx / 2, st, d, ntb, off);
         else if (c.pack && c.fuse_src) k_update_s_el2<R, X, true><<<c.s_grid, c.bx / 2, 0, st>>>(d, ntb, off);
         else if (c.pack) k_update_s_el2<R, X><<<c.s_grid, c.bx / 2, 0, st>>>(d, ntb, off);
         else k_update_s_el<R, X><<<c.tile_grid, c.bx, 0, st>>>(d, ntb, off);

@@ -40,11 +40,14 @@ SMALL = [
 IDS = [f"{c['nx']}x{c['ny']}-fd{c['fdorder']}-L{c.get('L', 0)}-{k}" for k, c in enumerate(SMALL)]
 
 
-@pytest.mark.parametrize("way", ["default", "injected"])
+@pytest.mark.parametrize("way", ["default", "paired", "injected"])
 @pytest.mark.parametrize("case", SMALL, ids=IDS)
 def test_small_batch_steps_bitexact(monkeypatch, case, way):
-    """The default way, and with the surface, receivers and sources in kernels of their own; the
-    launch count tells a folded step (two launches) from the other."""
+    """The default way (the small kernels for L = 0), without the small kernels, and with the surface,
+    receivers and sources in kernels of their own; the launch count tells a folded step (two
+    launches) from the last."""
+    if way != "default":
+        monkeypatch.setenv("DN_SMALL", "0")
     if way == "injected":
         monkeypatch.setenv("DN_SRC_IN_KERNEL", "0")
     p, model, src, rec = _case(nt=120, **case)
@@ -55,8 +58,11 @@ def test_small_batch_steps_bitexact(monkeypatch, case, way):
     _check(p, model, src, rec, s, (0, 1))
 
 
-def test_small_batch_of_unequal_shots():
-    """Shots of different sizes and step counts; a second run repeats the first."""
+@pytest.mark.parametrize("rows", [1, 3])
+def test_small_batch_of_unequal_shots(monkeypatch, rows):
+    """Shots of different sizes and step counts, tiles of one row and of three; a second run repeats
+    the first."""
+    monkeypatch.setenv("DN_TILE", f"128x{rows}")
     cases = [_case(nx=131, ny=37, nt=90, seed=1), _case(nx=300, ny=21, nt=140, styp=2, seed=2),
              _case(nx=64, ny=64, nt=61, free_surf=0, seed=5)]
     pairs = [gpu_shot(*c) for c in cases]
