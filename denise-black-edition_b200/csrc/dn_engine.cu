@@ -172,6 +172,7 @@ struct dn_shot {
     int nsnap = 0, zch = 16, bx = 128, tiles_x = 0, tiles = 0;
     int kern = DN_KERN_PAIRED;     // stencil kernel variant (the batch runs its first shot's)
     bool auto_rows = false;        // tile rows chosen per batch (batch_rows)
+    bool auto_stencil = false;     // the same for a shot whose snapshots keep tiles of zch rows
     bool rec_dup = false;          // two receivers share a cell
     // fused elastic step (DN_KERN_FUSED on an eligible shot): the second set of fields and
     // velocity CPML memory (inside dstate, so zeroed with it) and the tile rows
@@ -623,8 +624,8 @@ static void tile_choice(const dn_params *p, int &bx, int &zch, int &variant, boo
     if (deflt) *deflt = !from_rule;
 }
 
-// Rows per tile of a batch of shots that keep their tiles open (no snapshots, no
-// rule, no DN_TILE): the best of 1, 2, 4, 8 rows depends on the cells of the whole
+// Rows per tile of a batch of shots that keep their tiles open (no rule, no
+// DN_TILE; snapshots have tiles of their own, see eff_rows): the best of 1, 2, 4, 8 rows depends on the cells of the whole
 // batch, not of one shot.  Measured on a B200 (600 x 300 and 2000 x 600 grids, 1-32
 // shots, forward): one row up to 1.3 M cells (one 600 x 300 shot: 24.0 us a step
 // against 40.8 at 4 rows), two up to 5 M, four up to 16 M (viscoelastic: 30 M), eight
@@ -810,6 +811,7 @@ extern "C" int dn_shot_create(dn_model *m, const dn_acq *acq, dn_shot **out)
     bool deflt = false;
     tile_choice(p, s->bx, s->zch, s->kern, &deflt);
     s->auto_rows = deflt && !p->store_snapshots;
+    s->auto_stencil = deflt && p->store_snapshots;
     shot_counts(p, s->bx, s->zch, s->tiles_x, s->tiles, s->nsnap);
     s->acc64 = p->grad_accum == DN_ACC_F64;
 
@@ -1002,7 +1004,11 @@ static bool runs_fused(const dn_shot *s, int mode) { return s->fz && (mode == 0 
 // rows per tile of shot s in a batch configured as c
 static int eff_rows(const dn_shot *s, const LaunchCfg *c)
 {
-    return (c && c->auto_zch > 0 && s->auto_rows) ? c->auto_zch : s->zch;
+    if (!c || c->auto_zch <= 0) return s->zch;
+    if (s->auto_rows) return c->auto_zch;
+    // a gradient's batch beside its snapshots: shorter tiles while it is small, as for the others,
+    // never taller (128 x 8 ran 8 % slower there)
+    return s->auto_stencil ? std::min(c->auto_zch, s->zch) : s->zch;
 }
 static int eff_tiles(const dn_shot *s, const LaunchCfg *c)
 {
@@ -1048,6 +1054,8 @@ static Inst make_inst(const dn_shot *s, int mode, const LaunchCfg *c)
     I.zch = eff_rows(s, c);
     I.tiles_x = s->tiles_x;
     I.tiles = eff_tiles(s, c);
+    I.s_zch = s->zch;
+    I.s_tiles = s->tiles;
     I.store = (mode == 0) && p.store_snapshots && s->nsnap > 0;
     I.dtinv = std::max(p.dtinv, 1);
     I.nsnap = s->nsnap;
@@ -1312,7 +1320,7 @@ static int check_batch(dn_shot *const *shots, int n, int mode, LaunchCfg &c, con
     if (pk) c.pack = !c.tma && strcmp(pk, "0") != 0;
     c.any_surf = c.any_src_s = c.any_store = c.any_adj = c.any_rec = false;
     c.any_fused = c.any_plain = false;
-    int maxtiles = 0, maxsrc = 1, maxnx = 1, maxtr = 1, maxft = 1;
+    int maxtiles = 0, maxsnap = 1, maxsrc = 1, maxnx = 1, maxtr = 1, maxft = 1;
     {
         long long cells = 0;
         for (int k = 0; k < n; k++)
@@ -1335,6 +1343,7 @@ static int check_batch(dn_shot *const *shots, int n, int mode, LaunchCfg &c, con
                     return dn_fail(DN_ENOTSUP, "moment-tensor sources are not supported in the adjoint pass");
         }
         maxtiles = std::max(maxtiles, eff_tiles(s, &c));
+        maxsnap = std::max(maxsnap, s->tiles);
         if (runs_fused(s, m)) {
             c.any_fused = true;
             const int fwd = fz_width(s->p.fdorder / 2);
@@ -1350,6 +1359,7 @@ static int check_batch(dn_shot *const *shots, int n, int mode, LaunchCfg &c, con
         if (m == 1) c.any_adj = true;
     }
     c.tile_grid = dim3(maxtiles, n);
+    c.snap_grid = dim3(maxsnap, n);
     c.fgrid = dim3(maxft, n);
     // pipelined velocity kernel (DN_VPIPE=1): strips of VP_W columns, about four CTAs per
     // resident slot (148 SMs x 3) over the batch, at least 32 rows tall (DN_VPIPE_ROWS sets it)

@@ -39,7 +39,8 @@ namespace dn {
 struct Inst {
     int nx, ny, nt, pitch;
     int fw, free_surf, L, mode;       // mode: 0 forward, 1 adjoint, 2 objective
-    int zch, tiles_x, tiles;          // rows per tile, tiles across, total tiles
+    int zch, tiles_x, tiles;          // rows per tile, tiles across, total tiles of the stencil kernels
+    int s_zch, s_tiles;               // rows per tile, total tiles of the snapshots (as wide)
     int store;                        // mode 0: store snapshots
     int dtinv, nsnap, snap_prec, acc64, eprecond;
     int seismo;                       // SEISMO
@@ -1462,7 +1463,7 @@ __global__ void k_seismo(const Inst *__restrict__ insts, const int *__restrict__
 // ===========================================================================
 // Snapshot encoding.  Snapshot k holds the five fields of psv.c:246-298
 // (vxp1, vyp1, sxx, syy, sxy) of forward step 1 + k*DTINV.  Each field of
-// each tile (blockDim.x x zch cells) carries its own power-of-two scale so
+// each tile (blockDim.x x s_zch cells) carries its own power-of-two scale so
 // FP16 keeps ~11 significant bits over the whole dynamic range.
 // ===========================================================================
 __device__ __forceinline__ float warp_max(float v)
@@ -1513,7 +1514,7 @@ template <int PREC, int ZR>
 __device__ __forceinline__ void snap_store_regs(const Inst &I, int k, int b, int i, int j0, int nrow, bool in, float *red)
 {
     const long long P = I.pitch;
-    const long long tile_cells = (long long)blockDim.x * I.zch;
+    const long long tile_cells = (long long)blockDim.x * I.s_zch;
     const float *src[5] = {I.vxp1, I.vyp1, I.sxx, I.syy, I.sxy};
     float v[5][ZR], am[5];
 #pragma unroll
@@ -1536,7 +1537,7 @@ __device__ __forceinline__ void snap_store_regs(const Inst &I, int k, int b, int
     for (int f = 0; f < 5; f++) {
         float m = 0.0f;
         for (int q = 0; q < nw; q++) m = fmaxf(m, red[f * 8 + q]);
-        const long long slot = ((long long)k * 5 + f) * I.tiles + b;
+        const long long slot = ((long long)k * 5 + f) * I.s_tiles + b;
         const float sc = pow2_scale(m);
         const float inv = 1.0f / sc;   // exact: power of two
         if (threadIdx.x == 0) I.snap_scale[slot] = sc;
@@ -1556,15 +1557,15 @@ static __global__ void k_snap_store(const Inst *__restrict__ insts, const int *_
     const int k = (nt - 1) / I.dtinv - I.snap_base;
     if (k < 0 || k >= I.nsnap) return;
     const int b = blockIdx.x;
-    if (b >= I.tiles) return;
+    if (b >= I.s_tiles) return;
     __shared__ float red[5 * 8];   // five maxima of up to 8 warps
     const int tx = b % I.tiles_x, tz = b / I.tiles_x;
     const int i = tx * blockDim.x + threadIdx.x + 1;
-    const int j0 = tz * I.zch + 1;
-    const int nrow = min(I.zch, I.ny - j0 + 1);
+    const int j0 = tz * I.s_zch + 1;
+    const int nrow = min(I.s_zch, I.ny - j0 + 1);
     const bool in = i <= I.nx;
     const long long P = I.pitch;
-    const long long tile_cells = (long long)blockDim.x * I.zch;
+    const long long tile_cells = (long long)blockDim.x * I.s_zch;
     const float *src[5] = {I.vxp1, I.vyp1, I.sxx, I.syy, I.sxy};
     if (I.eprecond == 1 || I.eprecond == 3) {
         for (int r = 0; r < nrow && in; r++) {
@@ -1573,14 +1574,14 @@ static __global__ void k_snap_store(const Inst *__restrict__ insts, const int *_
             I.Ws[w] = __fadd_rn(I.Ws[w], __fadd_rn(__fmul_rn(I.vx[o], I.vx[o]), __fmul_rn(I.vy[o], I.vy[o])));
         }
     }
-    if (I.snap_prec != DN_SNAP_F32 && I.zch <= 4) {   // the default tile height: 20 values in registers
+    if (I.snap_prec != DN_SNAP_F32 && I.s_zch <= 4) {   // the default tile height: 20 values in registers
         if (I.snap_prec == DN_SNAP_F16)
             snap_store_regs<DN_SNAP_F16, 4>(I, k, b, i, j0, nrow, in, red);
         else
             snap_store_regs<DN_SNAP_BF16, 4>(I, k, b, i, j0, nrow, in, red);
         return;
     }
-    if (I.snap_prec != DN_SNAP_F32 && I.zch <= 8) {
+    if (I.snap_prec != DN_SNAP_F32 && I.s_zch <= 8) {
         if (I.snap_prec == DN_SNAP_F16)
             snap_store_regs<DN_SNAP_F16, 8>(I, k, b, i, j0, nrow, in, red);
         else
@@ -1588,7 +1589,7 @@ static __global__ void k_snap_store(const Inst *__restrict__ insts, const int *_
         return;
     }
     for (int f = 0; f < 5; f++) {
-        const long long slot = ((long long)k * 5 + f) * I.tiles + b;
+        const long long slot = ((long long)k * 5 + f) * I.s_tiles + b;
         const long long base = slot * tile_cells;
         if (I.snap_prec == DN_SNAP_F32) {
             float *dst = (float *)I.snap + base;
@@ -1677,8 +1678,8 @@ template <int PREC, typename A>
 __device__ __forceinline__ void correlate_tile(const Inst &I, int k, int b, int i, int j0, int nrow)
 {
     const long long P = I.pitch;
-    const long long T = I.tiles;
-    const long long tc = (long long)blockDim.x * I.zch;   // cells per tile slot
+    const long long T = I.s_tiles;
+    const long long tc = (long long)blockDim.x * I.s_zch;   // cells per tile slot
     const long long s0 = (long long)k * 5 * T + b;        // slot of the first of the five fields
     const size_t esz = PREC == DN_SNAP_F32 ? 4 : 2;
     const char *sp = (const char *)I.snap + (s0 * tc + threadIdx.x) * esz;
@@ -1752,12 +1753,12 @@ static __global__ void __launch_bounds__(256, DN_CORR_MINB) k_correlate(const In
     const int k = (nf - 1) / I.dtinv - I.snap_base;
     if (k < 0 || k >= I.nsnap) return;
     const int b = blockIdx.x;
-    if (b >= I.tiles) return;
+    if (b >= I.s_tiles) return;
     const int tx = b % I.tiles_x, tz = b / I.tiles_x;
     const int i = tx * blockDim.x + threadIdx.x + 1;
     if (i > I.nx) return;
-    const int j0 = tz * I.zch + 1;
-    const int nrow = min(I.zch, I.ny - j0 + 1);
+    const int j0 = tz * I.s_zch + 1;
+    const int nrow = min(I.s_zch, I.ny - j0 + 1);
     if (I.snap_prec == DN_SNAP_F16)
         correlate_prec<DN_SNAP_F16>(I, k, b, i, j0, nrow);
     else if (I.snap_prec == DN_SNAP_BF16)

@@ -13,6 +13,7 @@ namespace dn {
 
 struct LaunchCfg {
     dim3 tile_grid, src_grid, surf_grid, rec_grid;
+    dim3 snap_grid;   // the snapshots' tiles per instance
     dim3 s_grid;      // grid of the stress kernels: rec_blocks receiver blocks, then the tiles
     int bx;
     int auto_zch;     // rows per tile of the shots whose tiles the batch chooses (0: their own)

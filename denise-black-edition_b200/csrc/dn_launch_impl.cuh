@@ -92,12 +92,12 @@ void launch_step_R(const LaunchCfg &c, cudaStream_t st, const Inst *d, const int
     }
     MARK(6);
     if (c.any_store) {
-        k_snap_store<<<c.tile_grid, c.bx, 0, st>>>(d, ntb, off);
+        k_snap_store<<<c.snap_grid, c.bx, 0, st>>>(d, ntb, off);
         nl++;
     }
     MARK(7);
     if (c.any_adj) {
-        k_correlate<<<c.tile_grid, c.bx, 0, st>>>(d, ntb, off);
+        k_correlate<<<c.snap_grid, c.bx, 0, st>>>(d, ntb, off);
         nl++;
     }
     MARK(8);
