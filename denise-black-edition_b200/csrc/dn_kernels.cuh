@@ -478,8 +478,11 @@ __global__ void __launch_bounds__(128, DN_V2_MINB) k_update_v2(const Inst *__res
     for (int j = j0; j <= j1; j++) {
         const long long o = (long long)j * P + i0;
         // the lines row j + 1 reads first (its new z-stencil rows and its own-row operands) are
-        // requested into L1 now; every address stays inside the padded planes (rows up to ny + R + 1)
-        {
+        // requested into L1 now; every address stays inside the padded planes (rows up to ny + R + 1).
+        // Not in small batches at FDORDER 12, whose short tiles find 13 rows a column in L1 anyway
+        // (three 1501 x 747 shots: 45.4 ms with, 44.4 without; 16 shots of 2000 x 600 at FDORDER 8:
+        // 161.4 with, 170.9 without)
+        if constexpr (!(SRC && R == 6)) {
             constexpr int D = DN_PF_ROWS;   // rows ahead; D <= HZ - R keeps the addresses inside the planes
             pf_l1(I.syy + o + (R + D) * P);
             pf_l1(I.sxy + o + (R - 1 + D) * P);
@@ -1073,7 +1076,7 @@ __global__ void __launch_bounds__(128, DN_S2_MINB) k_update_s_el2(const Inst *__
     const int jsurf = SRC && I.surf_s ? R + 1 : 0;   // the last row with an image above the surface
     for (int j = j0; j <= j1; j++) {
         const long long o = (long long)j * P + i0;
-        {
+        if constexpr (!(SRC && R == 6)) {
             constexpr int D = DN_PF_ROWS;
             pf_l1(I.vx + o + (R + D) * P);
             pf_l1(I.vy + o + (R - 1 + D) * P);
