@@ -125,7 +125,10 @@ extern "C" int dn_device_trim(int device)
     cudaGetDevice(&cur);
     cudaError_t e = cudaSetDevice(device);
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
-    if (e == cudaSuccess) release_cached(device);
+    if (e == cudaSuccess) {
+        release_cached(device);
+        dn_grad_scratch_release(device);
+    }
     cudaSetDevice(cur);
     if (e != cudaSuccess) return dn_fail(DN_EDEVICE, "dn_device_trim(%d): %s", device, cudaGetErrorString(e));
     return DN_OK;

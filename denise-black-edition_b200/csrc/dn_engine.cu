@@ -994,7 +994,7 @@ static void *acc_ptr(const dn_shot *s, int k)
     return b + 3 * a + (k - 3) * w;
 }
 
-constexpr long long SMALL_CELLS = 1300000;   // cells of a batch below which the small kernels run
+constexpr long long SMALL_CELLS = 300000;   // cells of a batch below which the small kernels run
 // source cells per shot up to which the stencil kernels apply the forward sources themselves
 constexpr int SRC_IN_KERNEL = DN_SRC_CELLS;
 
@@ -1416,16 +1416,19 @@ static int check_batch(dn_shot *const *shots, int n, int mode, LaunchCfg &c, con
     // kernels of large batches the extra row test cost more than the launches (8000 x 2000 with
     // checkpoints 6 % slower), so those keep the surface and receiver kernels
     c.fold = c.fuse_src;
-    // one-row elastic batches (below 1.3 M cells): the kernels built for the shortest chain of
-    // dependent round trips; they take a column or row to lie in one CPML side at most, and every
-    // instance through the separate kernels.  Above, resident blocks count for more than the chain:
-    // three 1501 x 747 shots (3.4 M cells) took 62.0 ms with them and 45.4 with the paired kernels.
+    // the smallest elastic batches: the kernels built for the shortest chain of dependent round
+    // trips; they take a column or row to lie in one CPML side at most, and every instance through
+    // the separate kernels.  The line lies at two waves of their blocks (8 of 64 threads per SM,
+    // 128 cells each): one 600 x 300 shot (0.18 M cells) 22.5 ms with them and 30.4 with the paired
+    // kernels, a gradient of four 601 x 301 shots (0.72 M) 47.9 and 41.9, three 1501 x 747 shots
+    // (3.4 M) 62.0 and 45.4.  Not in run queues (modes): their streams fill the chip together, and
+    // a waiting overlapped launch would hold blocks that another queue could use.
     // DN_SMALL=0 / 1: never / whatever the size
     {
         const char *sm = getenv("DN_SMALL");
         long long cells = 0;
         for (int k = 0; k < n; k++) cells += (long long)shots[k]->p.nx * shots[k]->p.ny;
-        c.small = c.fuse_src && c.L == 0 && !c.any_fused && (sm ? strcmp(sm, "0") != 0 : cells < SMALL_CELLS);
+        c.small = c.fuse_src && c.L == 0 && !c.any_fused && !modes && (sm ? strcmp(sm, "0") != 0 : cells < SMALL_CELLS);
         for (int k = 0; k < n; k++)
             if (shots[k]->p.nx < 2 * shots[k]->p.fw || shots[k]->p.ny < 2 * shots[k]->p.fw || shots[k]->bx > 128)
                 c.small = false;
@@ -2434,7 +2437,7 @@ struct GradScratch {
     bool ok = false;
 };
 static std::mutex g_grad_mu;
-static std::map<int, GradScratch> g_grad_scratch;   // two chunks per device, allocated on first use
+static std::map<int, GradScratch> g_grad_scratch;   // two chunks per device, allocated on first use, released by dn_device_trim
 
 // out[e - e0] = in[j * nx + i] for e = i * ny + j in [e0, e1); blockIdx.x: 32 columns from column c0
 template <typename T>
@@ -2498,6 +2501,20 @@ static int grad_scratch(int device, GradScratch **out)
         }
     g.ok = true;
     return DN_OK;
+}
+
+// gives a device's chunks back (dn_device_trim)
+void dn_grad_scratch_release(int device)
+{
+    std::lock_guard<std::mutex> lk(g_grad_mu);
+    auto it = g_grad_scratch.find(device);
+    if (it == g_grad_scratch.end()) return;
+    for (int k = 0; k < 2; k++) {
+        if (it->second.d[k]) cudaFree(it->second.d[k]);
+        if (it->second.h[k]) cudaFreeHost(it->second.h[k]);
+        if (it->second.ev[k]) cudaEventDestroy(it->second.ev[k]);
+    }
+    g_grad_scratch.erase(it);
 }
 
 extern "C" int dn_model_get_gradient(const dn_model *m, float *g_vp, float *g_vs, float *g_rho)

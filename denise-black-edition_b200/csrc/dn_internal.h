@@ -57,6 +57,7 @@ inline cudaError_t dn_malloc(T **p, size_t bytes)
 }
 void dn_free(void *p);
 size_t dn_pool_idle_bytes(int device);
+void dn_grad_scratch_release(int device);   // the gradient read-back's buffers of a device
 #endif
 
 #ifdef __cplusplus

@@ -1,5 +1,5 @@
-// Velocity and elastic stress updates of the smallest batches (one-row tiles, up to about one
-// tile per resident thread group on the chip).
+// Velocity and elastic stress updates of the smallest batches (one-row tiles, up to about two
+// tiles per resident block on the chip).
 //
 // The step of such a batch is bound by the chain of dependent memory round trips of one thread,
 // each to L2 and back, not by bytes or instructions.  So every block copies its instance
@@ -13,7 +13,7 @@
 //
 // Measured against the folded paired kernels (2000 steps): 300 x 150, FDORDER 4: 27.3 -> 13.0 ms;
 // 600 x 300, FDORDER 8: 30.1 -> 22.5 ms (its 1500 blocks are a quarter more than the 8 resident
-// on each SM); the gradient of four 601 x 301 shots of 500 steps 51.9 -> 48.0 ms.  128 registers
+// on each SM).  128 registers
 // (8 blocks of 64 threads per SM) because with 80 or 64 the operands spill (300 x 150: 17.3 and
 // 16.9 ms); requesting the lines into L1 first and loading late was slower still (27.6 ms).
 #pragma once
