@@ -120,14 +120,14 @@ size_t dn_pool_idle_bytes(int device)
 
 extern "C" int dn_device_trim(int device)
 {
-    std::lock_guard<std::mutex> lk(g_mu);
     int cur = 0;
     cudaGetDevice(&cur);
     cudaError_t e = cudaSetDevice(device);
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     if (e == cudaSuccess) {
+        dn_grad_scratch_release(device);   // into the cache
+        std::lock_guard<std::mutex> lk(g_mu);
         release_cached(device);
-        dn_grad_scratch_release(device);
     }
     cudaSetDevice(cur);
     if (e != cudaSuccess) return dn_fail(DN_EDEVICE, "dn_device_trim(%d): %s", device, cudaGetErrorString(e));

@@ -12,6 +12,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <new>
 #include <string>
 #include <thread>
 #include <vector>
@@ -2481,39 +2482,72 @@ static void place(float *dst, const float *src, size_t n)
         if (th[k].joinable()) th[k].join();
 }
 
-static int grad_scratch(int device, GradScratch **out)
+static void grad_scratch_free(GradScratch &g)
+{
+    for (int k = 0; k < 2; k++) {
+        dn_free(g.d[k]);
+        if (g.h[k]) cudaFreeHost(g.h[k]);
+        if (g.ev[k]) cudaEventDestroy(g.ev[k]);
+    }
+    g = GradScratch();
+}
+
+// false: no memory for the chunks, even with the library's cached blocks released (dn_malloc)
+static bool grad_scratch(int device, GradScratch **out)
 {
     GradScratch &g = g_grad_scratch[device];
     *out = &g;
-    if (g.ok) return DN_OK;
+    if (g.ok) return true;
     for (int k = 0; k < 2; k++)
-        if (cudaMalloc(&g.d[k], GRAD_CHUNK * 4) != cudaSuccess ||
+        if (dn_malloc(&g.d[k], GRAD_CHUNK * 4) != cudaSuccess ||
             cudaMallocHost(&g.h[k], GRAD_CHUNK * 4) != cudaSuccess ||
             cudaEventCreateWithFlags(&g.ev[k], cudaEventDisableTiming) != cudaSuccess) {
             cudaGetLastError();
-            for (int q = 0; q < 2; q++) {
-                if (g.d[q]) cudaFree(g.d[q]);
-                if (g.h[q]) cudaFreeHost(g.h[q]);
-                if (g.ev[q]) cudaEventDestroy(g.ev[q]);
-            }
-            g = GradScratch();
-            return dn_fail(DN_ENOMEM, "dn_model_get_gradient: scratch allocation failed");
+            grad_scratch_free(g);
+            return false;
         }
     g.ok = true;
+    return true;
+}
+
+// the same without scratch: blocks of rows copied as they lie, the order restored on the host.
+// For a device (or pinned memory) without 16 MB left, where a gradient already computed must
+// still come out.
+static int gradient_by_host(const dn_model *m, float *const outs[3])
+{
+    const int nx = m->p.nx, ny = m->p.ny;
+    const size_t n = (size_t)nx * ny, esz = m->grad64 ? 8 : 4;
+    const int rows = (int)std::max<long long>(1, std::min<long long>(ny, GRAD_CHUNK / nx));
+    std::vector<char> h;
+    try {
+        h.resize((size_t)rows * nx * esz);
+    } catch (const std::bad_alloc &) {
+        return dn_fail(DN_ENOMEM, "dn_model_get_gradient: %zu bytes of host memory", (size_t)rows * nx * esz);
+    }
+    for (int c = 0; c < 3; c++) {
+        if (!outs[c]) continue;
+        for (int j0 = 0; j0 < ny; j0 += rows) {
+            const int r = std::min(rows, ny - j0);
+            CU(cudaMemcpy(h.data(), (const char *)m->dgrad + (c * n + (size_t)j0 * nx) * esz, (size_t)r * nx * esz,
+                          cudaMemcpyDeviceToHost));
+            for (int i = 0; i < nx; i++)
+                for (int j = 0; j < r; j++) {
+                    const size_t w = (size_t)j * nx + i;
+                    outs[c][(size_t)i * ny + j0 + j] = m->grad64 ? (float)((double *)h.data())[w] : ((float *)h.data())[w];
+                }
+        }
+    }
     return DN_OK;
 }
 
-// gives a device's chunks back (dn_device_trim)
+// gives a device's chunks back (dn_device_trim, before it takes the block cache's lock: the chunks
+// come from that cache, so g_grad_mu is taken first everywhere)
 void dn_grad_scratch_release(int device)
 {
     std::lock_guard<std::mutex> lk(g_grad_mu);
     auto it = g_grad_scratch.find(device);
     if (it == g_grad_scratch.end()) return;
-    for (int k = 0; k < 2; k++) {
-        if (it->second.d[k]) cudaFree(it->second.d[k]);
-        if (it->second.h[k]) cudaFreeHost(it->second.h[k]);
-        if (it->second.ev[k]) cudaEventDestroy(it->second.ev[k]);
-    }
+    grad_scratch_free(it->second);
     g_grad_scratch.erase(it);
 }
 
@@ -2524,10 +2558,9 @@ extern "C" int dn_model_get_gradient(const dn_model *m, float *g_vp, float *g_vs
     const long long n = (long long)nx * ny;
     CU(cudaSetDevice(m->device));
     std::lock_guard<std::mutex> lk(g_grad_mu);
-    GradScratch *g;
-    const int st = grad_scratch(m->device, &g);
-    if (st) return st;
     float *outs[3] = {g_vp, g_vs, g_rho};
+    GradScratch *g;
+    if (!grad_scratch(m->device, &g)) return gradient_by_host(m, outs);
     struct Part {
         float *dst;
         size_t n;

@@ -22,3 +22,37 @@ def test_gradient_readback_order(nx, ny, acc):
     m.set_gradient(*g)
     for a, b in zip(m.gradient(), g):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("idle", [False, True])
+def test_gradient_readback_on_a_full_device(idle):
+    """No device memory left for the read-back's chunks: the gradient still comes out, by the
+    blocks that the library keeps idle (idle) or without any device memory."""
+    import torch
+
+    from denise_b200 import _lib, synth
+
+    p = synth.c0_params(nx=1201, ny=1801, nt=10, fw=0, store_snapshots=1, grad_accum=_lib.ACC_F64)
+    one = np.ones((p.nx, p.ny), np.float32)
+    m = dn.Model(p, 3000 * one, 1700 * one, 2000 * one)
+    rng = np.random.default_rng(3)
+    g = [rng.standard_normal((p.nx, p.ny)).astype(np.float32) for _ in range(3)]
+    m.set_gradient(*g)
+    m.gradient()   # its kernels are loaded before the device is full
+    dn.device_trim(0)
+    if idle:
+        dn.Model(p, 3000 * one, 1700 * one, 2000 * one).close()
+    full, size = [], 64 << 30
+    while size >= 1 << 20:
+        try:
+            full.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+        except torch.cuda.OutOfMemoryError:
+            size //= 2
+    try:
+        assert torch.cuda.mem_get_info(0)[0] < 8 << 20   # a chunk does not fit
+        got = m.gradient()
+    finally:
+        full.clear()
+        torch.cuda.empty_cache()
+    for a, b in zip(got, g):
+        np.testing.assert_array_equal(a, b)
