@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "dn_internal.h"
+#include "dn_perdev.h"
 #include "dn_precond.h"
 #include "dn_launch.cuh"
 #include "dn_materials.cuh"
@@ -2437,8 +2438,7 @@ struct GradScratch {
     cudaEvent_t ev[2] = {nullptr, nullptr};
     bool ok = false;
 };
-static std::mutex g_grad_mu;
-static std::map<int, GradScratch> g_grad_scratch;   // two chunks per device, allocated on first use, released by dn_device_trim
+static PerDevice<GradScratch> g_grad_scratch;   // two chunks per device, allocated on first use, released by dn_device_trim
 
 // out[e - e0] = in[j * nx + i] for e = i * ny + j in [e0, e1); blockIdx.x: 32 columns from column c0
 template <typename T>
@@ -2493,10 +2493,8 @@ static void grad_scratch_free(GradScratch &g)
 }
 
 // false: no memory for the chunks, even with the library's cached blocks released (dn_malloc)
-static bool grad_scratch(int device, GradScratch **out)
+static bool grad_scratch(GradScratch &g)
 {
-    GradScratch &g = g_grad_scratch[device];
-    *out = &g;
     if (g.ok) return true;
     for (int k = 0; k < 2; k++)
         if (dn_malloc(&g.d[k], GRAD_CHUNK * 4) != cudaSuccess ||
@@ -2541,14 +2539,12 @@ static int gradient_by_host(const dn_model *m, float *const outs[3])
 }
 
 // gives a device's chunks back (dn_device_trim, before it takes the block cache's lock: the chunks
-// come from that cache, so g_grad_mu is taken first everywhere)
+// come from that cache, so the scratch's lock is taken first everywhere)
 void dn_grad_scratch_release(int device)
 {
-    std::lock_guard<std::mutex> lk(g_grad_mu);
-    auto it = g_grad_scratch.find(device);
-    if (it == g_grad_scratch.end()) return;
-    grad_scratch_free(it->second);
-    g_grad_scratch.erase(it);
+    PerDevice<GradScratch>::Slot &slot = g_grad_scratch.at(device);
+    std::lock_guard<std::mutex> lk(slot.mu);
+    grad_scratch_free(slot.value);
 }
 
 extern "C" int dn_model_get_gradient(const dn_model *m, float *g_vp, float *g_vs, float *g_rho)
@@ -2557,10 +2553,11 @@ extern "C" int dn_model_get_gradient(const dn_model *m, float *g_vp, float *g_vs
     const int nx = m->p.nx, ny = m->p.ny;
     const long long n = (long long)nx * ny;
     CU(cudaSetDevice(m->device));
-    std::lock_guard<std::mutex> lk(g_grad_mu);
     float *outs[3] = {g_vp, g_vs, g_rho};
-    GradScratch *g;
-    if (!grad_scratch(m->device, &g)) return gradient_by_host(m, outs);
+    PerDevice<GradScratch>::Slot &slot_dev = g_grad_scratch.at(m->device);
+    std::lock_guard<std::mutex> lk(slot_dev.mu);
+    GradScratch *const g = &slot_dev.value;
+    if (!grad_scratch(*g)) return gradient_by_host(m, outs);
     struct Part {
         float *dst;
         size_t n;
