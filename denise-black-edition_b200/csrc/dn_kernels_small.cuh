@@ -259,7 +259,6 @@ __global__ void __launch_bounds__(64, 8) k_update_s_el2_small(const Inst *__rest
     xf.coefs(I, i0, I.K_x, I.a_x, I.b_x, I.K_xh, I.a_xh, I.b_xh);
     const bool srcs = I.fsrc_s && small_source(I, i0, two, j0, j1, nt);
     const int jsurf = I.surf_s ? R + 1 : 0;   // the last row with an image above the surface
-    if (jsurf && j0 == 1 && xf.in[0]) pf_l1(I.psi_vxxs + xf.h[0]);
     const float dhi = I.dhi_el;
     for (int j = j0; j <= j1; j++) {
         const long long o = (long long)j * P + i0;
@@ -278,6 +277,7 @@ __global__ void __launch_bounds__(64, 8) k_update_s_el2_small(const Inst *__rest
         }
         const float2 s_xx = ldw2(I.sxx + o), s_yy = ldw2(I.syy + o), s_xy = ldw2(I.sxy + o);
         xf.load(I, j, I.psi_vxx, I.psi_vyx);
+        if (jsurf && j == 1 && xf.in[0]) pf_l1(I.psi_vxxs + xf.h[0]);   // for the surface condition below
         zf.load(I.psi_vyy, I.psi_vxy, two);
         float2 vxx = MUL2<X>(bc2(I.hc[1]), SUB2<X>(pair_at<R, KC>(lc, R), pair_at<R, KC>(lc, R - 1)));
         float2 vyx = MUL2<X>(bc2(I.hc[1]), SUB2<X>(pair_at<R, KD>(ld, R), pair_at<R, KD>(ld, R - 1)));
