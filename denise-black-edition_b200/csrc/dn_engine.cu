@@ -84,6 +84,7 @@ static std::mutex g_dev_mu;
 static std::map<int, DevState> g_dev;
 static thread_local double g_last_ms = 0.0;
 static thread_local long long g_last_launches = 0;
+static thread_local int g_last_route = 0;
 
 static int dev_state(int device, DevState **out)
 {
@@ -1275,6 +1276,7 @@ struct Batch {
     cudaGraphExec_t exec = nullptr;
     int chunk = 0;
     long long launches_per_chunk = 0;
+    int route = 0;
 };
 static std::mutex g_batch_mu;
 static std::vector<Batch *> g_batches;   // small cache of captured graphs
@@ -1450,6 +1452,13 @@ static int check_batch(dn_shot *const *shots, int n, int mode, LaunchCfg &c, con
     return DN_OK;
 }
 
+// dn_last_run_route of a batch configured as c
+static int route_of(const dn_shot *first, const LaunchCfg &c)
+{
+    return (c.pack ? DN_ROUTE_PAIRED : 0) | (c.small ? DN_ROUTE_SMALL : 0) | (c.fuse_src ? DN_ROUTE_SRC : 0) |
+           (c.fold ? DN_ROUTE_FOLD : 0) | (c.any_fused ? DN_ROUTE_FUSED : 0) | eff_rows(first, &c) << 8;
+}
+
 static int zero_for_run(dn_shot *s, int mode, cudaStream_t st)
 {
     CU(cudaMemsetAsync(s->dstate, 0, s->state_bytes, st));   // zero_denise_*_PSV
@@ -1610,6 +1619,7 @@ static int run_ckpt(dn_shot *const *shots, int n, int mode, double &ms_total, lo
     float ms = 0.0f;
     cudaEventElapsedTime(&ms, ds->ev0, ds->ev1);
     ms_total += ms;
+    g_last_route = route_of(s0, c);
     dn_free(d);
     if (le != cudaSuccess) return dn_fail(DN_EDEVICE, "kernel launch failed: %s", cudaGetErrorString(le));
     return st;
@@ -1690,6 +1700,7 @@ extern "C" int dn_run(dn_shot *const *shots, int n, int mode)
             return dn_fail(DN_EDEVICE, "graph instantiate failed: %s", cudaGetErrorString(e));
         }
         b->launches_per_chunk = nl;
+        b->route = route_of(shots[0], c);
         std::lock_guard<std::mutex> lk(g_batch_mu);
         if (g_batches.size() >= 8) {
             batch_free(g_batches.front());
@@ -1711,6 +1722,7 @@ extern "C" int dn_run(dn_shot *const *shots, int n, int mode)
     cudaEventElapsedTime(&ms, ds->ev0, ds->ev1);
     g_last_ms = ms;
     g_last_launches = b->launches_per_chunk * nchunks;
+    g_last_route = b->route;
     return st;
 }
 
@@ -1768,6 +1780,7 @@ static int run_direct(dn_shot *s, int mode, int nt0, int nt1, bool zero)
     cudaEventElapsedTime(&ms, ds->ev0, ds->ev1);
     g_last_ms = ms;
     g_last_launches = nl;
+    g_last_route = route_of(s, c);
     dn_free(d);
     if (le != cudaSuccess) return dn_fail(DN_EDEVICE, "kernel launch failed: %s", cudaGetErrorString(le));
     return st;
@@ -1794,6 +1807,8 @@ extern "C" int dn_last_run_stats(double *ms, long long *launches)
     if (launches) *launches = g_last_launches;
     return DN_OK;
 }
+
+extern "C" int dn_last_run_route(void) { return g_last_route; }
 
 // ---------------------------------------------------------------------------
 // run queues: continuous batching

@@ -377,6 +377,15 @@ def last_run_stats():
     return ms.value, nl.value
 
 
+ROUTES = (("paired", 1), ("small", 2), ("src", 4), ("fold", 8), ("fused", 16))   # DN_ROUTE_* bits
+
+
+def last_run_route():
+    """Names of the kernels the last run of this thread took (DN_ROUTE_*), and its stencil tiles' rows."""
+    r = lib.dn_last_run_route()
+    return {n for n, b in ROUTES if r & b}, r >> 8
+
+
 KERNEL_SLOTS = ("update_v", "inject_v", "update_s", "inject_s", "surface", "seismo", "snap_store", "correlate")
 
 

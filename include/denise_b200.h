@@ -327,6 +327,16 @@ int dn_shot_get_snapshot(const dn_shot *s, int k, int field, float *out);
  * around the time loop only) and the number of kernel launches it issued. */
 int dn_last_run_stats(double *device_ms, long long *launches);
 
+/* Which kernels the last dn_run / dn_run_plain / dn_run_steps of this thread took: the batch's size,
+ * sources, sections and free surfaces choose them, results do not depend on it.  DN_ROUTE_* bits, and
+ * the rows of the stencil tiles of its first shot from bit 8 up. */
+#define DN_ROUTE_PAIRED 1   /* two adjacent columns per thread */
+#define DN_ROUTE_SMALL 2    /* the kernels of the smallest elastic batches */
+#define DN_ROUTE_SRC 4      /* forward sources inside the stencil kernels */
+#define DN_ROUTE_FOLD 8     /* free surfaces and velocity receivers inside the stress kernels */
+#define DN_ROUTE_FUSED 16   /* some shot took the fused elastic step */
+int dn_last_run_route(void);
+
 /* calc_res() for LNORM = 2 (src/calc_res.c:306-445 residual, :514-568 misfit) on
  * the device.  syn_tm: synthetic section, time-major [nt][ntr] (the layout the
  * propagator records); obs: observed section [ntr][nt]; res (out): adjoint
