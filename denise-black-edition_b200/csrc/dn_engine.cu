@@ -1414,12 +1414,6 @@ static int check_batch(dn_shot *const *shots, int n, int mode, LaunchCfg &c, con
             }
         }
     }
-    // free surface and velocity receivers inside the same variants of the stress kernels: two of
-    // the four dependent launches of a step go, and a small batch's step is bound by them (one
-    // 600 x 300 shot 21.9 -> 15.0 us a step, one viscoelastic 2000 x 600 shot 75 -> 63 us); in the
-    // kernels of large batches the extra row test cost more than the launches (8000 x 2000 with
-    // checkpoints 6 % slower), so those keep the surface and receiver kernels
-    c.fold = c.fuse_src;
     // the smallest elastic batches: the kernels built for the shortest chain of dependent round
     // trips; they take a column or row to lie in one CPML side at most, and every instance through
     // the separate kernels.  The line lies at two waves of their blocks (8 of 64 threads per SM,
@@ -1437,13 +1431,30 @@ static int check_batch(dn_shot *const *shots, int n, int mode, LaunchCfg &c, con
             if (shots[k]->p.nx < 2 * shots[k]->p.fw || shots[k]->p.ny < 2 * shots[k]->p.fw || shots[k]->bx > 128)
                 c.small = false;
     }
-    c.rec_blocks = 0;
-    for (int k = 0; k < n; k++) {
-        const dn_shot *s = shots[k];
-        const int m = modes ? modes[k] : mode;
-        if (s->p.free_surf && !surf_in_stress(s, m, &c)) c.any_surf = true;
-        if (rec_in_stress(s, m, &c)) c.rec_blocks = std::max(1, std::min((maxtr + 127) / 128, 16));
-        else c.any_rec = true;
+    // free surface and velocity receivers inside the stress kernels of the same batches (their FOLD
+    // variants; the small kernels always can): two of the four dependent launches of a step go, and
+    // a small batch's step is bound by them (one 600 x 300 shot 21.9 -> 15.0 us a step, one
+    // viscoelastic 2000 x 600 shot 75 -> 63 us); in the kernels of large batches the extra row test
+    // cost more than the launches (8000 x 2000 with checkpoints 6 % slower).  Only where a launch
+    // goes: a batch that keeps both (no free surface and stress sections, say) would pay for the
+    // row test alone, up to 5 % at FDORDER 10
+    auto settle = [&] {   // what is left for k_surface_* and k_seismo; whether one of them goes
+        c.any_surf = c.any_rec = false;
+        c.rec_blocks = 0;
+        bool surf = false;
+        for (int k = 0; k < n; k++) {
+            const dn_shot *s = shots[k];
+            const int m = modes ? modes[k] : mode;
+            if (s->p.free_surf) (surf_in_stress(s, m, &c) ? surf : c.any_surf) = true;
+            if (rec_in_stress(s, m, &c)) c.rec_blocks = std::max(1, std::min((maxtr + 127) / 128, 16));
+            else c.any_rec = true;
+        }
+        return (surf && !c.any_surf) || !c.any_rec;
+    };
+    c.fold = c.fuse_src;
+    if (!settle() && c.fold && !c.small) {
+        c.fold = false;
+        settle();
     }
     c.s_grid = dim3(maxtiles + c.rec_blocks, n);
     c.src_grid = dim3((maxsrc + 127) / 128, n);

@@ -502,12 +502,12 @@ template <int LL>
 void launch_vi(const Inst *d, dim3 grid)
 {
     switch (FDORDER / 2) {
-    case 1: dn::k_update_s_vi<1, LL, true, false, true><<<grid, 128>>>(d, g.d_zero, 1); break;
-    case 2: dn::k_update_s_vi<2, LL, true, false, true><<<grid, 128>>>(d, g.d_zero, 1); break;
-    case 3: dn::k_update_s_vi<3, LL, true, false, true><<<grid, 128>>>(d, g.d_zero, 1); break;
-    case 4: dn::k_update_s_vi<4, LL, true, false, true><<<grid, 128>>>(d, g.d_zero, 1); break;
-    case 5: dn::k_update_s_vi<5, LL, true, false, true><<<grid, 128>>>(d, g.d_zero, 1); break;
-    default: dn::k_update_s_vi<6, LL, true, false, true><<<grid, 128>>>(d, g.d_zero, 1); break;
+    case 1: dn::k_update_s_vi<1, LL, true, false, false, true><<<grid, 128>>>(d, g.d_zero, 1); break;
+    case 2: dn::k_update_s_vi<2, LL, true, false, false, true><<<grid, 128>>>(d, g.d_zero, 1); break;
+    case 3: dn::k_update_s_vi<3, LL, true, false, false, true><<<grid, 128>>>(d, g.d_zero, 1); break;
+    case 4: dn::k_update_s_vi<4, LL, true, false, false, true><<<grid, 128>>>(d, g.d_zero, 1); break;
+    case 5: dn::k_update_s_vi<5, LL, true, false, false, true><<<grid, 128>>>(d, g.d_zero, 1); break;
+    default: dn::k_update_s_vi<6, LL, true, false, false, true><<<grid, 128>>>(d, g.d_zero, 1); break;
     }
 }
 

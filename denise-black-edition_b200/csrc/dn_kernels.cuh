@@ -1045,7 +1045,7 @@ __device__ __forceinline__ void vderiv2(const Inst &I, const float *hc, int i0, 
 
 
 // Paired-column elastic stress update (k_update_s_el for two columns per thread).
-template <int R, bool X, bool SRC = false>
+template <int R, bool X, bool SRC = false, bool FOLD = false>
 __global__ void __launch_bounds__(128, DN_S2_MINB) k_update_s_el2(const Inst *__restrict__ insts, const int *__restrict__ ntb, int off)
 {
     const Inst &I = insts[blockIdx.y];
@@ -1053,7 +1053,7 @@ __global__ void __launch_bounds__(128, DN_S2_MINB) k_update_s_el2(const Inst *__
     const int nt = *ntb + off - I.t0;   // the instance's own time step
     if (nt < 1 || nt > I.nt) return;
     int b = blockIdx.x;
-    if constexpr (SRC) {   // the first rec_blocks blocks record the receivers
+    if constexpr (FOLD) {   // the first rec_blocks blocks record the receivers
         b -= I.rec_blocks;
         if (b < 0) {
             record_velocities(I, nt, blockIdx.x, I.rec_blocks);
@@ -1073,7 +1073,7 @@ __global__ void __launch_bounds__(128, DN_S2_MINB) k_update_s_el2(const Inst *__
     for (int m = 1; m <= R; m++) hc[m] = I.hc[m];
     const float dhi = I.dhi_el;
     const bool srcs = SRC && I.fsrc_s && src_in_columns(I, i0, two, j0, j1);
-    const int jsurf = SRC && I.surf_s ? R + 1 : 0;   // the last row with an image above the surface
+    const int jsurf = FOLD && I.surf_s ? R + 1 : 0;   // the last row with an image above the surface
     for (int j = j0; j <= j1; j++) {
         const long long o = (long long)j * P + i0;
         if constexpr (!(SRC && R == 6)) {
@@ -1103,7 +1103,7 @@ __global__ void __launch_bounds__(128, DN_S2_MINB) k_update_s_el2(const Inst *__
             nsyy.y = F(DADD((double)s_yy.y, DADD((double)gdiv.y, DMUL(f2y, (double)vyy.y))));
         }
         if (srcs) src_explosive_pair(I, i0, two, j, nt, nsxx, nsyy);
-        if (SRC && j <= jsurf) {
+        if (FOLD && j <= jsurf) {
             if (j == 1) {
                 nsyy = make_float2(0.0f, 0.0f);
                 nsxx.x = surface_sxx_el_call<R, X>(I, i0, o, nsxx.x);
@@ -1124,14 +1124,14 @@ __global__ void __launch_bounds__(128, DN_S2_MINB) k_update_s_el2(const Inst *__
 // factors exactly as prepare_update_s_visc_PSV.c:52-62 forms them; the PRE
 // variant reads them prepared (Inst::pre_*), as the reference function takes them.
 // ===========================================================================
-template <int R, int L, bool X, bool SRC = false, bool PRE = false>
+template <int R, int L, bool X, bool SRC = false, bool FOLD = false, bool PRE = false>
 __global__ void __launch_bounds__(256, 3) k_update_s_vi(const Inst *__restrict__ insts, const int *__restrict__ ntb, int off)
 {
     const Inst &I = insts[blockIdx.y];
     const int nt = *ntb + off - I.t0;   // the instance's own time step
     if (nt < 1 || nt > I.nt) return;
     int b = blockIdx.x;
-    if constexpr (SRC) {   // the first rec_blocks blocks record the receivers
+    if constexpr (FOLD) {   // the first rec_blocks blocks record the receivers
         b -= I.rec_blocks;
         if (b < 0) {
             record_velocities(I, nt, blockIdx.x, I.rec_blocks);
@@ -1203,7 +1203,7 @@ __global__ void __launch_bounds__(256, 3) k_update_s_vi(const Inst *__restrict__
         }
     };
     const bool srcs = SRC && I.fsrc_s && src_in_columns(I, i, false, t.j0, t.j1);
-    const int jsurf = SRC && I.surf_s ? R + 1 : 0;   // the last row with an image above the surface
+    const int jsurf = FOLD && I.surf_s ? R + 1 : 0;   // the last row with an image above the surface
     fetch(t.j0);
     for (int j = t.j0; j <= t.j1; j++) {
         D.advance(j);
@@ -1269,7 +1269,7 @@ __global__ void __launch_bounds__(256, 3) k_update_s_vi(const Inst *__restrict__
             for (int c = 0; c < I.nsrc_cells; c++)
                 if (I.src_cell_j[c] == j && I.src_cell_i[c] == i)
                     fz_explosive(I, I.src_cell_start[c], I.src_cell_count[c], nt, fsxx, fsyy);
-        if (SRC && j <= jsurf) {
+        if (FOLD && j <= jsurf) {
             if (j == 1) {
                 fsyy = 0.0f;
 #pragma unroll

@@ -14,7 +14,7 @@ namespace dn {
 struct LaunchCfg {
     dim3 tile_grid, src_grid, surf_grid, rec_grid;
     dim3 snap_grid;   // the snapshots' tiles per instance
-    dim3 s_grid;      // grid of the stress kernels: rec_blocks receiver blocks, then the tiles
+    dim3 s_grid;      // grid of the folding stress kernels: rec_blocks receiver blocks, then the tiles
     int bx;
     int auto_zch;     // rows per tile of the shots whose tiles the batch chooses (0: their own)
     int R, L;
@@ -25,7 +25,7 @@ struct LaunchCfg {
     bool vpipe; // velocity update by the warp-specialised copy pipeline (k_update_v_pipe)
     dim3 vgrid; // its grid: strips of VP_W columns x vsh rows per instance
     int vsh;
-    bool fold;        // the stress kernels can take the free surface and the velocity receivers
+    bool fold;        // the stress kernels take free surfaces and velocity receivers (FOLD variants, small kernels)
     int rec_blocks;   // receiver blocks of their grid
     bool any_surf;    // k_surface_* still has work
     bool any_rec;     // k_seismo still has work

@@ -37,8 +37,9 @@ void launch_step_R(const LaunchCfg &c, cudaStream_t st, const Inst *d, const int
         if (c.tma)
             k_update_s_el_tma<R, X><<<c.tile_grid, TMA_W, pipe_smem_bytes<QS_EL>(slot_floats_s_el()), st>>>(d, ntb, off);
         else if (c.small) launch_pdl(k_update_s_el2_small<R, X>, c.s_grid, c.bx / 2, st, d, ntb, off);
-        else if (c.pack && c.fuse_src) k_update_s_el2<R, X, true><<<c.s_grid, c.bx / 2, 0, st>>>(d, ntb, off);
-        else if (c.pack) k_update_s_el2<R, X><<<c.s_grid, c.bx / 2, 0, st>>>(d, ntb, off);
+        else if (c.fold) k_update_s_el2<R, X, true, true><<<c.s_grid, c.bx / 2, 0, st>>>(d, ntb, off);
+        else if (c.pack && c.fuse_src) k_update_s_el2<R, X, true><<<c.tile_grid, c.bx / 2, 0, st>>>(d, ntb, off);
+        else if (c.pack) k_update_s_el2<R, X><<<c.tile_grid, c.bx / 2, 0, st>>>(d, ntb, off);
         else k_update_s_el<R, X><<<c.tile_grid, c.bx, 0, st>>>(d, ntb, off);
     } else if (c.tma) {
 #define DN_VI_TMA(LL)                                                                                          \
@@ -53,8 +54,9 @@ void launch_step_R(const LaunchCfg &c, cudaStream_t st, const Inst *d, const int
 #undef DN_VI_TMA
     } else {
 #define DN_VI(LL)                                                                                              \
-    (c.fuse_src ? k_update_s_vi<R, LL, X, true><<<c.s_grid, c.bx, 0, st>>>(d, ntb, off)                        \
-                : k_update_s_vi<R, LL, X><<<c.s_grid, c.bx, 0, st>>>(d, ntb, off))
+    (c.fold ? k_update_s_vi<R, LL, X, true, true><<<c.s_grid, c.bx, 0, st>>>(d, ntb, off)                      \
+     : c.fuse_src ? k_update_s_vi<R, LL, X, true><<<c.tile_grid, c.bx, 0, st>>>(d, ntb, off)                   \
+                  : k_update_s_vi<R, LL, X><<<c.tile_grid, c.bx, 0, st>>>(d, ntb, off))
         switch (c.L) {
         case 1: DN_VI(1); break;
         case 2: DN_VI(2); break;

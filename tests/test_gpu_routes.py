@@ -161,3 +161,30 @@ def test_receiver_counts_of_a_folded_batch(monkeypatch, L, way):
             np.testing.assert_array_equal(s.sections(comp), ref.sections(comp))
         for name, fid in (("vx", 0), ("vy", 1), ("sxx", 2), ("syy", 3), ("sxy", 4)):
             np.testing.assert_array_equal(s.field(fid), ref.field(fid), err_msg=name)
+
+
+@pytest.mark.parametrize("L", [0, 2])
+@pytest.mark.parametrize("shots,fold", [
+    (((1, 1, 1),), True), (((1, 4, 1),), True), (((0, 1, 1),), True),
+    (((0, 4, 1),), False),                   # neither launch goes
+    (((1, 4, 1), (1, 4, 5)), False),         # a moment tensor keeps k_surface_*, stress sections k_seismo
+    (((1, 1, 1), (1, 4, 5)), False),
+    (((1, 1, 1), (0, 4, 1)), True),          # k_surface_* goes
+    (((1, 1, 5), (0, 1, 1)), True),          # k_seismo goes
+])
+def test_folds_only_where_a_launch_goes(monkeypatch, shots, fold, L):
+    """Shots (free surface, SEISMO, source type) of one batch in the paired kernels: the variants
+    with the surface rows and receiver blocks run only if k_surface_* or k_seismo is spared."""
+    _take(monkeypatch, "paired")
+    cases = [_case(nx=131, ny=37, nt=80, L=L, free_surf=fs, styp=styp, seed=k) for k, (fs, _, styp) in enumerate(shots)]
+    cases = [(c[0].replace(seismo=se), *c[1:]) for c, (_, se, _) in zip(cases, shots)]
+    pairs = [gpu_shot(*c) for c in cases]
+    dn.run([s for _, s in pairs], dn.MODE_FORWARD)
+    assert ("fold" in dn.last_run_route()[0]) == fold
+    for c, (_, s) in zip(cases, pairs):
+        ref = O.Restatement(*c, "f")
+        ref.forward(store=False)
+        for comp in ((0, 1) if c[0].seismo == 1 else range(5)):
+            np.testing.assert_array_equal(s.sections(comp), ref.sections(comp))
+        for name, fid in (("vx", 0), ("vy", 1), ("sxx", 2), ("syy", 3), ("sxy", 4)):
+            np.testing.assert_array_equal(s.field(fid), ref.field(fid), err_msg=name)
