@@ -448,6 +448,17 @@ __device__ __forceinline__ float2 DIVH2(float2 a, bool fd, float DH, float rdh)
     return q1;
 }
 
+// Whether the paired kernels request the next row's lines ahead.  The batches of the SRC variants
+// (below 5 M cells) have tiles of one or two rows, so at most half of the rows have a next one in
+// their tile.  Step times without the requests over those with, 0.04 - 4.3 M cells, with and without
+// free surface, forward and gradients, elastic / viscoelastic (L 3): FDORDER 4 0.91 - 0.98 / 0.98 -
+// 0.99, FDORDER 10 0.90 - 0.99 / 0.98 - 1.00, FDORDER 12 0.94 - 0.99 / 0.98 - 1.00; but FDORDER 2
+// 0.94 - 1.04 / 0.99 - 1.01, FDORDER 6 0.94 - 1.01 / 0.99 - 1.01, FDORDER 8 0.95 - 1.00 / 0.98 -
+// 1.02, which keep them.  So do larger batches (16 shots of 2000 x 600 at FDORDER 8: 161 ms with,
+// 171 without).
+template <int R, bool SRC>
+constexpr bool row_prefetch = !(SRC && (R == 2 || R >= 5));
+
 // SRC: the variant that applies the forward sources of its cells (Inst::fsrc_v)
 template <int R, bool X, bool SRC = false>
 __global__ void __launch_bounds__(128, DN_V2_MINB) k_update_v2(const Inst *__restrict__ insts, const int *__restrict__ ntb, int off)
@@ -478,11 +489,8 @@ __global__ void __launch_bounds__(128, DN_V2_MINB) k_update_v2(const Inst *__res
     for (int j = j0; j <= j1; j++) {
         const long long o = (long long)j * P + i0;
         // the lines row j + 1 reads first (its new z-stencil rows and its own-row operands) are
-        // requested into L1 now; every address stays inside the padded planes (rows up to ny + R + 1).
-        // Not in small batches at FDORDER 12, whose short tiles find 13 rows a column in L1 anyway
-        // (three 1501 x 747 shots: 45.4 ms with, 44.4 without; 16 shots of 2000 x 600 at FDORDER 8:
-        // 161.4 with, 170.9 without)
-        if constexpr (!(SRC && R == 6)) {
+        // requested into L1 now; every address stays inside the padded planes (rows up to ny + R + 1)
+        if constexpr (row_prefetch<R, SRC>) {
             constexpr int D = DN_PF_ROWS;   // rows ahead; D <= HZ - R keeps the addresses inside the planes
             pf_l1(I.syy + o + (R + D) * P);
             pf_l1(I.sxy + o + (R - 1 + D) * P);
@@ -1076,7 +1084,7 @@ __global__ void __launch_bounds__(128, DN_S2_MINB) k_update_s_el2(const Inst *__
     const int jsurf = FOLD && I.surf_s ? R + 1 : 0;   // the last row with an image above the surface
     for (int j = j0; j <= j1; j++) {
         const long long o = (long long)j * P + i0;
-        if constexpr (!(SRC && R == 6)) {
+        if constexpr (row_prefetch<R, SRC>) {
             constexpr int D = DN_PF_ROWS;
             pf_l1(I.vx + o + (R + D) * P);
             pf_l1(I.vy + o + (R - 1 + D) * P);
