@@ -2458,13 +2458,18 @@ extern "C" int dn_shot_accumulate_gradient_ex(dn_shot *s, const dn_accum_opts *o
 // host, one strided element at a time, took 155 of the 289 ms of a checkpointed 8000 x 2000
 // gradient of 96 steps (the whole call now 133 ms).
 // ---------------------------------------------------------------------------
-constexpr long long GRAD_CHUNK = 2 << 20;   // floats of one chunk (8 MB)
+constexpr long long GRAD_CHUNK = 2 << 20;   // floats of one chunk at most (8 MB)
+// cells up to which the host restores the order after a single copy: there three kernels and copies
+// take longer (64 x 48: 52 us against 41; 300 x 150: 84 against 207)
+constexpr long long GRAD_HOST = 4096;
 struct GradScratch {
     float *d[2] = {nullptr, nullptr}, *h[2] = {nullptr, nullptr};
     cudaEvent_t ev[2] = {nullptr, nullptr};
-    bool ok = false;
+    long long n = 0;   // floats of a chunk
 };
-static PerDevice<GradScratch> g_grad_scratch;   // two chunks per device, allocated on first use, released by dn_device_trim
+// two chunks per device, as large as the largest gradient so far asks for (16 MB of pinned memory
+// take 10 ms to get, 200 times what reading a small gradient takes), released by dn_device_trim
+static PerDevice<GradScratch> g_grad_scratch;
 
 // out[e - e0] = in[j * nx + i] for e = i * ny + j in [e0, e1); blockIdx.x: 32 columns from column c0
 template <typename T>
@@ -2518,46 +2523,51 @@ static void grad_scratch_free(GradScratch &g)
     g = GradScratch();
 }
 
-// false: no memory for the chunks, even with the library's cached blocks released (dn_malloc)
-static bool grad_scratch(GradScratch &g)
+// false: no memory for chunks of n floats, even with the library's cached blocks released (dn_malloc)
+static bool grad_scratch(GradScratch &g, long long n)
 {
-    if (g.ok) return true;
+    if (g.n >= n) return true;
+    grad_scratch_free(g);
     for (int k = 0; k < 2; k++)
-        if (dn_malloc(&g.d[k], GRAD_CHUNK * 4) != cudaSuccess ||
-            cudaMallocHost(&g.h[k], GRAD_CHUNK * 4) != cudaSuccess ||
+        if (dn_malloc(&g.d[k], n * 4) != cudaSuccess || cudaMallocHost(&g.h[k], n * 4) != cudaSuccess ||
             cudaEventCreateWithFlags(&g.ev[k], cudaEventDisableTiming) != cudaSuccess) {
             cudaGetLastError();
             grad_scratch_free(g);
             return false;
         }
-    g.ok = true;
+    g.n = n;
     return true;
 }
 
 // the same without scratch: blocks of rows copied as they lie, the order restored on the host.
-// For a device (or pinned memory) without 16 MB left, where a gradient already computed must
-// still come out.
+// For the smallest gradients, and for a device (or pinned memory) without 16 MB left, where a
+// gradient already computed must still come out.
 static int gradient_by_host(const dn_model *m, float *const outs[3])
 {
     const int nx = m->p.nx, ny = m->p.ny;
     const size_t n = (size_t)nx * ny, esz = m->grad64 ? 8 : 4;
+    const bool whole = n <= (size_t)GRAD_HOST;   // all three in one copy
     const int rows = (int)std::max<long long>(1, std::min<long long>(ny, GRAD_CHUNK / nx));
+    const size_t bytes = (whole ? 3 * n : (size_t)rows * nx) * esz;
     std::vector<char> h;
     try {
-        h.resize((size_t)rows * nx * esz);
+        h.resize(bytes);
     } catch (const std::bad_alloc &) {
-        return dn_fail(DN_ENOMEM, "dn_model_get_gradient: %zu bytes of host memory", (size_t)rows * nx * esz);
+        return dn_fail(DN_ENOMEM, "dn_model_get_gradient: %zu bytes of host memory", bytes);
     }
+    if (whole) CU(cudaMemcpy(h.data(), m->dgrad, bytes, cudaMemcpyDeviceToHost));
     for (int c = 0; c < 3; c++) {
         if (!outs[c]) continue;
         for (int j0 = 0; j0 < ny; j0 += rows) {
             const int r = std::min(rows, ny - j0);
-            CU(cudaMemcpy(h.data(), (const char *)m->dgrad + (c * n + (size_t)j0 * nx) * esz, (size_t)r * nx * esz,
-                          cudaMemcpyDeviceToHost));
+            if (!whole)
+                CU(cudaMemcpy(h.data(), (const char *)m->dgrad + (c * n + (size_t)j0 * nx) * esz,
+                              (size_t)r * nx * esz, cudaMemcpyDeviceToHost));
+            const char *p = h.data() + (whole ? c * n * esz : 0);
             for (int i = 0; i < nx; i++)
                 for (int j = 0; j < r; j++) {
                     const size_t w = (size_t)j * nx + i;
-                    outs[c][(size_t)i * ny + j0 + j] = m->grad64 ? (float)((double *)h.data())[w] : ((float *)h.data())[w];
+                    outs[c][(size_t)i * ny + j0 + j] = m->grad64 ? (float)((const double *)p)[w] : ((const float *)p)[w];
                 }
         }
     }
@@ -2580,10 +2590,11 @@ extern "C" int dn_model_get_gradient(const dn_model *m, float *g_vp, float *g_vs
     const long long n = (long long)nx * ny;
     CU(cudaSetDevice(m->device));
     float *outs[3] = {g_vp, g_vs, g_rho};
+    if (n <= GRAD_HOST) return gradient_by_host(m, outs);
     PerDevice<GradScratch>::Slot &slot_dev = g_grad_scratch.at(m->device);
     std::lock_guard<std::mutex> lk(slot_dev.mu);
     GradScratch *const g = &slot_dev.value;
-    if (!grad_scratch(*g)) return gradient_by_host(m, outs);
+    if (!grad_scratch(*g, std::min(n, GRAD_CHUNK))) return gradient_by_host(m, outs);
     struct Part {
         float *dst;
         size_t n;

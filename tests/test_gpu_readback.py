@@ -24,6 +24,30 @@ def test_gradient_readback_order(nx, ny, acc):
         np.testing.assert_array_equal(a, b)
 
 
+@pytest.mark.parametrize("acc", ["f32", "f64"])
+@pytest.mark.parametrize("nx,ny", [(64, 64), (241, 17), (300, 150), (1201, 1801), (33, 200)])
+def test_readback_takes_no_more_memory_than_the_gradient(nx, ny, acc):
+    """The first read-back of a gradient costs what that gradient needs, not the largest chunks; sizes
+    on both sides of the line to the single copy, and larger and smaller ones in turn."""
+    from denise_b200 import _lib, synth
+
+    p = synth.c0_params(nx=nx, ny=ny, nt=10, fw=0, store_snapshots=1,
+                        grad_accum=_lib.ACC_F64 if acc == "f64" else _lib.ACC_F32)
+    one = np.ones((nx, ny), np.float32)
+    m = dn.Model(p, 3000 * one, 1700 * one, 2000 * one)
+    rng = np.random.default_rng(ny)
+    g = [rng.standard_normal((nx, ny)).astype(np.float32) for _ in range(3)]
+    m.set_gradient(*g)
+    m.gradient()
+    dn.device_trim(0)
+    free = dn.device_memory(0)[0]
+    got = m.gradient()
+    taken = free - dn.device_memory(0)[0]
+    assert taken <= 2 * min(4 * nx * ny, 8 << 20) + (4 << 20), taken   # two chunks, in the driver's 2 MB steps
+    for a, b in zip(got, g):
+        np.testing.assert_array_equal(a, b)
+
+
 @pytest.mark.parametrize("idle", [False, True])
 def test_gradient_readback_on_a_full_device(idle):
     """No device memory left for the read-back's chunks: the gradient still comes out, by the
