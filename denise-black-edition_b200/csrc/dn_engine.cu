@@ -1414,23 +1414,6 @@ static int check_batch(dn_shot *const *shots, int n, int mode, LaunchCfg &c, con
             }
         }
     }
-    // the smallest elastic batches: the kernels built for the shortest chain of dependent round
-    // trips; they take a column or row to lie in one CPML side at most, and every instance through
-    // the separate kernels.  The line lies at two waves of their blocks (8 of 64 threads per SM,
-    // 128 cells each): one 600 x 300 shot (0.18 M cells) 22.5 ms with them and 30.4 with the paired
-    // kernels, a gradient of four 601 x 301 shots (0.72 M) 47.9 and 41.9, three 1501 x 747 shots
-    // (3.4 M) 62.0 and 45.4.  Not in run queues (modes): their streams fill the chip together, and
-    // a waiting overlapped launch would hold blocks that another queue could use.
-    // DN_SMALL=0 / 1: never / whatever the size
-    {
-        const char *sm = getenv("DN_SMALL");
-        long long cells = 0;
-        for (int k = 0; k < n; k++) cells += (long long)shots[k]->p.nx * shots[k]->p.ny;
-        c.small = c.fuse_src && c.L == 0 && !c.any_fused && !modes && (sm ? strcmp(sm, "0") != 0 : cells < SMALL_CELLS);
-        for (int k = 0; k < n; k++)
-            if (shots[k]->p.nx < 2 * shots[k]->p.fw || shots[k]->p.ny < 2 * shots[k]->p.fw || shots[k]->bx > 128)
-                c.small = false;
-    }
     // free surface and velocity receivers inside the stress kernels of the same batches (their FOLD
     // variants; the small kernels always can): two of the four dependent launches of a step go, and
     // a small batch's step is bound by them (one 600 x 300 shot 21.9 -> 15.0 us a step, one
@@ -1451,8 +1434,34 @@ static int check_batch(dn_shot *const *shots, int n, int mode, LaunchCfg &c, con
         }
         return (surf && !c.any_surf) || !c.any_rec;
     };
+    c.small = false;
     c.fold = c.fuse_src;
-    if (!settle() && c.fold && !c.small) {
+    const bool spared = settle();
+    // the smallest elastic batches: the kernels built for the shortest chain of dependent round
+    // trips; they take a column or row to lie in one CPML side at most, and every instance through
+    // the separate kernels.  The line lies at two waves of their blocks (8 of 64 threads per SM,
+    // 128 cells each): one 600 x 300 shot (0.18 M cells) 22.4 ms with them and 30.4 with the paired
+    // kernels, a gradient of four 601 x 301 shots (0.72 M) 47.9 and 41.9, three 1501 x 747 shots
+    // (3.4 M) 62.0 and 45.4.  Below it they are 1.00 to 2.7 times as fast up to FDORDER 10; at
+    // FDORDER 12 0.88 to 1.12 times beyond one wave of blocks, and where nothing is folded the line
+    // lies there, an eighth of a second wave included (all sections: four 200 x 150 shots, 1200
+    // blocks, 1.11 times, sixteen 100 x 90, 1440 blocks, 0.94, five 250 x 200, 2000 blocks, 0.90).
+    // Not in run queues (modes): their streams fill the chip together, and the serving mix takes
+    // 219 ms with and without them.  DN_SMALL=0 / 1: never / whatever the size
+    {
+        const char *sm = getenv("DN_SMALL");
+        long long cells = 0, blocks = 0;
+        for (int k = 0; k < n; k++) {
+            cells += (long long)shots[k]->p.nx * shots[k]->p.ny;
+            blocks += eff_tiles(shots[k], &c);
+        }
+        const bool below = cells < SMALL_CELLS && (c.R < 6 || spared || blocks <= 9 * 148);
+        c.small = c.fuse_src && c.L == 0 && !c.any_fused && !modes && (sm ? strcmp(sm, "0") != 0 : below);
+        for (int k = 0; k < n; k++)
+            if (shots[k]->p.nx < 2 * shots[k]->p.fw || shots[k]->p.ny < 2 * shots[k]->p.fw || shots[k]->bx > 128)
+                c.small = false;
+    }
+    if (!spared && c.fold && !c.small) {
         c.fold = false;
         settle();
     }
