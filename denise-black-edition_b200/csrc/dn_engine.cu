@@ -1019,17 +1019,17 @@ static int eff_tiles(const dn_shot *s, const LaunchCfg *c)
     return ((s->p.nx + s->bx - 1) / s->bx) * ((s->p.ny + z - 1) / z);
 }
 
-// whether the stress kernel can take over the free surface of shot s: not when a source that
-// k_inject_s adds afterwards sits in row 1 (the surface condition there starts from the sum), not
-// for moment tensors (they change sxy in two rows), and not when the images reach below the grid
+// whether the stress kernel can take over the free surface of shot s: not when an adjoint pressure
+// that k_inject_s adds afterwards lies in row 1 (the surface condition there starts from the sum;
+// forward explosive sources are in the stress kernel itself where it folds), not for moment tensors
+// (they change sxy in two rows), and not when the images reach below the grid
 static bool surf_in_stress(const dn_shot *s, int mode, const LaunchCfg *c)
 {
     if (!c || !c->fold || !s->p.free_surf || runs_fused(s, mode)) return false;
     if (s->p.ny < s->p.fdorder / 2 + 1) return false;
     if (mode == 1)
         return s->p.quelltypb < 4 || std::find(s->rec_j.begin(), s->rec_j.end(), 1) == s->rec_j.end();
-    if (s->quelltyp_last == 5) return false;
-    return c->fuse_src || s->quelltyp_last != 1 || std::find(s->src_j.begin(), s->src_j.end(), 1) == s->src_j.end();
+    return s->quelltyp_last != 5;
 }
 // whether the stress kernel's receiver blocks record shot s: the velocities only (SEISMO 2-4 need
 // the stresses after the sources and the surface, and stay with k_seismo)

@@ -1298,8 +1298,8 @@ __global__ void __launch_bounds__(256, 3) k_update_s_vi(const Inst *__restrict__
 // pressure source psource.c:41-53 (mode 1, QUELLTYPB >= 4) and the moment
 // tensor source msource.c:27-41 (QUELLTYP == 5, forward modes).
 // ===========================================================================
-// a stress source added below a surface that the stress kernel has already mirrored: the image
-// row of syy follows (rows 2 to R + 1; shots with such a source in row 1 keep the surface kernel)
+// an adjoint pressure added below a surface that the stress kernel has already mirrored: the image
+// row of syy follows (rows 2 to R + 1; shots with one in row 1 keep the surface kernel)
 __device__ __forceinline__ void inject_image(const Inst &I, int j, long long o, float syy)
 {
     if (I.surf_s && j >= 2 && j <= I.ord + 1) I.syy[o - 2 * (j - 1) * (long long)I.pitch] = -syy;
@@ -1345,7 +1345,6 @@ static __global__ void k_inject_s(const Inst *__restrict__ insts, const int *__r
             }
             I.sxx[o] = sxx;
             I.syy[o] = syy;
-            inject_image(I, I.src_cell_j[c], o, syy);
         }
     } else if (I.quelltyp_last == 5) {
         // neighbouring moment-tensor sources touch overlapping cells: one thread, list order

@@ -25,7 +25,7 @@ struct LaunchCfg {
     bool vpipe; // velocity update by the warp-specialised copy pipeline (k_update_v_pipe)
     dim3 vgrid; // its grid: strips of VP_W columns x vsh rows per instance
     int vsh;
-    bool fold;        // the stress kernels take free surfaces and velocity receivers (FOLD variants, small kernels)
+    bool fold;        // (only with fuse_src) the stress kernels take free surfaces and velocity receivers
     int rec_blocks;   // receiver blocks of their grid
     bool any_surf;    // k_surface_* still has work
     bool any_rec;     // k_seismo still has work
