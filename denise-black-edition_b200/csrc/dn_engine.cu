@@ -1418,9 +1418,10 @@ static int check_batch(dn_shot *const *shots, int n, int mode, LaunchCfg &c, con
     // variants; the small kernels always can): two of the four dependent launches of a step go, and
     // a small batch's step is bound by them (one 600 x 300 shot 21.9 -> 15.0 us a step, one
     // viscoelastic 2000 x 600 shot 75 -> 63 us); in the kernels of large batches the extra row test
-    // cost more than the launches (8000 x 2000 with checkpoints 6 % slower).  Only where a launch
-    // goes: a batch that keeps both (no free surface and stress sections, say) would pay for the
-    // row test alone, up to 5 % at FDORDER 10
+    // cost more than the launches (8000 x 2000 with checkpoints 6 % slower, eight 2000 x 600 shots up
+    // to 5 %; two 2500 x 1000 shots, 5.0 M cells, 5-8 % faster).  Only where a launch goes: a batch
+    // that keeps both (no free surface and stress sections, say) would pay for the row test alone,
+    // up to 5 % at FDORDER 10
     auto settle = [&] {   // what is left for k_surface_* and k_seismo; whether one of them goes
         c.any_surf = c.any_rec = false;
         c.rec_blocks = 0;
@@ -1440,7 +1441,7 @@ static int check_batch(dn_shot *const *shots, int n, int mode, LaunchCfg &c, con
     // the smallest elastic batches: the kernels built for the shortest chain of dependent round
     // trips; they take a column or row to lie in one CPML side at most, and every instance through
     // the separate kernels.  The line lies at two waves of their blocks (8 of 64 threads per SM,
-    // 128 cells each): one 600 x 300 shot (0.18 M cells) 22.4 ms with them and 30.4 with the paired
+    // 128 cells each): one 600 x 300 shot (0.18 M cells) 22.2 ms with them and 30.4 with the paired
     // kernels, a gradient of four 601 x 301 shots (0.72 M) 47.9 and 41.9, three 1501 x 747 shots
     // (3.4 M) 62.0 and 45.4.  Below it they are 1.00 to 2.7 times as fast up to FDORDER 10; at
     // FDORDER 12 0.88 to 1.12 times beyond one wave of blocks, and where nothing is folded the line

@@ -11,9 +11,10 @@
 // profiles) and waits for the predecessor before the first field.  Arithmetic and its order are
 // those of the paired kernels, so results are the same bits.
 //
-// Measured against the folded paired kernels (2000 steps): 300 x 150, FDORDER 4: 27.3 -> 13.0 ms;
-// 600 x 300, FDORDER 8: 30.1 -> 22.5 ms (its 1500 blocks are a quarter more than the 8 resident
-// on each SM).  128 registers
+// Measured against the folded paired kernels (2000 steps): 300 x 150, FDORDER 4: 27.3 -> 13.1 ms;
+// 600 x 300, FDORDER 8: 30.1 -> 22.2 ms (its 1500 blocks are a quarter more than the 8 resident
+// on each SM).  At 600 x 300 an SM issues in 28 % of its cycles and a warp waits 4.6 (velocity) and
+// 5.7 (stress) issue slots for loads per instruction, DRAM and L2 far from their rates.  128 registers
 // (8 blocks of 64 threads per SM) because with 80 or 64 the operands spill (300 x 150: 17.3 and
 // 16.9 ms); requesting the lines into L1 first and loading late was slower still (27.6 ms).
 #pragma once
