@@ -1444,9 +1444,10 @@ static int check_batch(dn_shot *const *shots, int n, int mode, LaunchCfg &c, con
     // 128 cells each): one 600 x 300 shot (0.18 M cells) 22.2 ms with them and 30.4 with the paired
     // kernels, a gradient of four 601 x 301 shots (0.72 M) 47.9 and 41.9, three 1501 x 747 shots
     // (3.4 M) 62.0 and 45.4.  Below it they are 1.00 to 2.7 times as fast up to FDORDER 10; at
-    // FDORDER 12 0.88 to 1.12 times beyond one wave of blocks, and where nothing is folded the line
-    // lies there, an eighth of a second wave included (all sections: four 200 x 150 shots, 1200
-    // blocks, 1.11 times, sixteen 100 x 90, 1440 blocks, 0.94, five 250 x 200, 2000 blocks, 0.90).
+    // FDORDER 12 0.88 to 1.12 times beyond one wave of blocks, and for several shots of which nothing
+    // is folded the line lies there, an eighth of a second wave included (all sections: four 200 x
+    // 150 shots, 1200 blocks, 1.11 times, sixteen 100 x 90, 1440 blocks, 0.94, five 250 x 200, 2000
+    // blocks, 0.90; single shots of 1500 to 2500 blocks 0.97 to 1.02, in direct launches 1.13).
     // Not in run queues (modes): their streams fill the chip together, and the serving mix takes
     // 219 ms with and without them.  DN_SMALL=0 / 1: never / whatever the size
     {
@@ -1456,7 +1457,7 @@ static int check_batch(dn_shot *const *shots, int n, int mode, LaunchCfg &c, con
             cells += (long long)shots[k]->p.nx * shots[k]->p.ny;
             blocks += eff_tiles(shots[k], &c);
         }
-        const bool below = cells < SMALL_CELLS && (c.R < 6 || spared || blocks <= 9 * 148);
+        const bool below = cells < SMALL_CELLS && (c.R < 6 || spared || n == 1 || blocks <= 9 * 148);
         c.small = c.fuse_src && c.L == 0 && !c.any_fused && !modes && (sm ? strcmp(sm, "0") != 0 : below);
         for (int k = 0; k < n; k++)
             if (shots[k]->p.nx < 2 * shots[k]->p.fw || shots[k]->p.ny < 2 * shots[k]->p.fw || shots[k]->bx > 128)

@@ -55,17 +55,17 @@ def test_route_of_a_batch(monkeypatch, nx, ny, L, fw, nsrc, env, small, src, row
     assert (("small" in names), ("src" in names), got) == (small, src, rows), names
 
 
-@pytest.mark.parametrize("fdorder,ny,seismo,small", [
-    (12, 333, 4, True), (12, 334, 4, False),     # 4 x 333 blocks: nine for each of 148 SMs
-    (12, 334, 1, True), (10, 334, 4, True)])
-def test_route_past_one_wave_of_blocks(fdorder, ny, seismo, small):
-    """FDORDER 12 without folded work leaves the small kernels soon after one wave of their blocks."""
+@pytest.mark.parametrize("fdorder,ny,shots,seismo,small", [
+    (12, 166, 2, 4, True), (12, 167, 2, 4, False),     # 4 x 166 x 2 of at most 9 x 148 blocks
+    (12, 167, 2, 1, True), (10, 167, 2, 4, True), (12, 334, 1, 4, True)])
+def test_route_past_one_wave_of_blocks(fdorder, ny, shots, seismo, small):
+    """FDORDER 12 shots without folded work leave the small kernels soon after one wave of their blocks."""
     p = synth.c0_params(nx=500, ny=ny, nt=4, fw=10, fdorder=fdorder, free_surf=0, seismo=seismo)
     one = np.ones((500, ny), np.float32)
     m = dn.Model(p, 3000 * one, 1700 * one, 2000 * one)
-    s = dn.Shot(m, np.array([50], np.int32), np.array([40], np.int32), np.ones((1, 4), np.float32),
-                np.array([60], np.int32), np.array([40], np.int32))
-    dn.run([s], dn.MODE_FORWARD)
+    at = [np.array([k], np.int32) for k in (50, 60, 40)]
+    batch = [dn.Shot(m, at[0], at[2], np.ones((1, 4), np.float32), at[1], at[2]) for _ in range(shots)]
+    dn.run(batch, dn.MODE_FORWARD)
     assert ("small" in dn.last_run_route()[0]) == small
 
 
